@@ -7,16 +7,28 @@
 // phase is swept by the whole grid with a grid barrier after it; the dense coarsest level
 // (at most a few thousand unknowns) is one GEMV with its precomputed inverse, a warp per row.
 //
-// PCG (FP64 vectors, scaled system A^ = D^-1/2 A D^-1/2):
-//   z = V(r);  beta = (r,z)/(r,z)_old;  c = (w,z)/(w,w) (singular systems: remove the
-//   null-vector component w = D^1/2 1 from z);  p = z - c w + beta p;
-//   q = A^ z + beta q  (A^ w = 0, so q = A^ p without a second SpMV), with A^ z evaluated as
-//   D^-1/2 [sum_j a_ij (u_j - u_i) + (sum_j a_ij) u_i], u = D^-1/2 z, FP32 a_ij, FP64 sums
-//   (the level-0 cycle works on the unscaled A and returns u directly, reading the same
-//   FP32 a_ij and columns);
-//   alpha = (r,z)/(p,q);  y += alpha p;  r -= alpha q.
+// PCG (FP64 vectors, on A itself; in exact arithmetic the same iterates as on D^-1/2 A D^-1/2):
+//   u = V(r);  beta = (r,u)/(r,u)_old;  c = (d,u)/(1,d) (singular systems: remove the constant
+//   from u, d the diagonal);  p = u - c + beta p;
+//   q = A u + beta q  (A 1 = 0, so q = A p without a second SpMV), with A u evaluated as
+//   sum_j a_ij (u_j - u_i) + (sum_j a_ij) u_i, FP32 a_ij (those of the cycle), FP64 sums;
+//   alpha = (r,u)/(p,q);  y += alpha p;  r -= alpha q.
 // The recurrence residual is confirmed against the true FP64 residual (FP64 values) before
-// returning; stopping rule ||b - A x|| <= max(rtol ||b||, atol) in the unscaled norm.
+// returning; stopping rule ||b - A x|| <= max(rtol ||b||, atol).
+//
+// What bounds k_pcg_amg is the chain of loads inside each of its 15 or so phases per
+// iteration, not bytes: 148 CTAs sweep 10^3 to 10^6 rows between two grid barriers of 1.3 us.
+// So (1) every CTA owns a contiguous block of slices of each level, and keeps their values,
+// columns and slice bounds in shared memory for the whole solve, as far as 200 KB go (finest
+// level first, which five phases of an iteration read): a phase's chain is one gather, and no
+// matrix byte crosses L2 again; slices past that stream from global memory in the same loop;
+// (2) eight gathers of a row are in flight; (3) the level descriptors are kernel parameters;
+// (4) the sums of the PCG ride on the barrier (sync_sum).  Per iteration, against sweeps that
+// read the matrices from global memory, two gathers in flight on a row's last columns:
+// 183 -> 96 us on the 400x400x2 film (level-0 sweeps 12-21 -> 6-8 us, product 18 -> 9.5,
+// update 13 -> 6; the restriction, the prolongation and the dense level, 9-12 us each, read
+// 12-25 MB through L2), 150 -> 80 us on the union of 64 boxes (375,280 nodes), 48 -> 26 us on
+// the 20x20x5 box, where a phase is 2-4 us, 1.3 of it the barrier.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -101,32 +113,28 @@ __global__ void k_to_float_rows(const double* __restrict__ a, float* __restrict_
   b[e] = j < n ? static_cast<float>(a[i * n + j]) : 0.0f;
 }
 
-__global__ void k_f32_to_f16(int64_t n, const float* __restrict__ a, __half* __restrict__ b) {
-  const int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (e < n) b[e] = __float2half_rn(a[e]);
-}
-
 }  // namespace
 
 void AmgDevice::upload(const AmgHost& h, cudaStream_t s, const int64_t* sp0, const int32_t* col0, const float* val0,
-                       int64_t nslices0, int nrep) {
+                       int64_t nslices0, int nrep, int grid) {
   reps = nrep;
   nlev = static_cast<int>(h.lv.size());
   n0 = h.lv[0].A.n;
   nc = h.lv.back().A.n;
   A.clear(); P.clear(); rrp.clear(); rcol.clear();
-  val.clear(); pval.clear(); rval.clear(); dinv.clear(); vec.clear(); val16.clear();
+  val.clear(); pval.clear(); rval.clear(); dinv.clear(); vec.clear();
   A.resize(nlev); P.resize(nlev); rrp.resize(nlev); rcol.resize(nlev);
-  val.resize(nlev); pval.resize(nlev); rval.resize(nlev); dinv.resize(nlev); vec.resize(nlev); val16.resize(nlev);
-  // FP16 values for the cycle's sweeps (tuning option: half the value bytes of every sweep;
-  // the PCG product keeps the FP32 values)
-  const char* e16 = std::getenv("SPX_AMG_FP16");
-  const bool fp16 = e16 && std::atoi(e16) != 0;
+  val.resize(nlev); pval.resize(nlev); rval.resize(nlev); dinv.resize(nlev); vec.resize(nlev);
   sizes.assign(nlev, 0);
   nnz.assign(nlev, 0);
   pnnz.assign(nlev, 0);
   rnnz.assign(nlev, 0);
-  std::vector<AmgLevelDev> d(nlev);
+  SPX_CHECK(nlev <= AMG_MAX_LEVELS, "too many AMG levels");
+  std::vector<AmgLevelDev>& d = lv;
+  d.assign(nlev, AmgLevelDev{});
+  need.assign(nlev, 0);
+  cnt.assign(nlev, 0);
+  res.assign(nlev, AmgResident{-1, 0, 0, 0, 0, 0});
   for (int l = 0; l < nlev; ++l) {
     const AmgHostLevel& L = h.lv[l];
     sizes[l] = L.A.n;
@@ -151,13 +159,14 @@ void AmgDevice::upload(const AmgHost& h, cudaStream_t s, const int64_t* sp0, con
     if (l + 1 == nlev) break;  // dense coarsest: vectors only
     HostSell hs, hp;
     std::vector<float> v, vp;
-    int64_t vlen = 0;
+    std::vector<int64_t> sph;
     if (l == 0 && sp0) {
       D.nslices = nslices0;
       D.sp = sp0;
       D.col = col0;
       D.val = val0;
-      SPX_CUDA(cudaMemcpyAsync(&vlen, sp0 + nslices0, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      sph.resize(nslices0 + 1);
+      SPX_CUDA(cudaMemcpyAsync(sph.data(), sp0, sph.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       SPX_CUDA(cudaStreamSynchronize(s));
     } else {
       csr_to_sell(L.A, hs, v);
@@ -167,14 +176,13 @@ void AmgDevice::upload(const AmgHost& h, cudaStream_t s, const int64_t* sp0, con
       D.sp = A[l].slice_ptr.p;
       D.col = A[l].col.p;
       D.val = val[l].p;
-      vlen = static_cast<int64_t>(v.size());
+      sph = hs.slice_ptr;
     }
-    D.val16 = nullptr;
-    if (fp16 && vlen > 0) {
-      val16[l].alloc(vlen);
-      k_f32_to_f16<<<grid_for(vlen, 256), 256, 0, s>>>(vlen, D.val, val16[l].p);
-      SPX_LAUNCH_CHECK();
-      D.val16 = val16[l].p;
+    // slices and entries of the largest CTA block of this level (slices [ns c / G, ns (c+1) / G))
+    for (int c = 0; c < grid; ++c) {
+      const int64_t a = D.nslices * c / grid, e = D.nslices * (c + 1) / grid;
+      cnt[l] = std::max(cnt[l], e - a);
+      need[l] = std::max(need[l], sph[e] - sph[a]);
     }
     csr_to_sell(L.P, hp, vp);
     P[l].upload(hp, s);
@@ -199,7 +207,6 @@ void AmgDevice::upload(const AmgHost& h, cudaStream_t s, const int64_t* sp0, con
     D.delta = static_cast<float>(0.5 * (b - a));
     D.sigma = static_cast<float>((b + a) / (b - a));
   }
-  lv.upload(d, s);
   // coarsest inverse: FP64 Gauss-Jordan on the device, stored FP32
   {
     DevBuf<double> M, colk;
@@ -220,7 +227,7 @@ void AmgDevice::upload(const AmgHost& h, cudaStream_t s, const int64_t* sp0, con
 }
 
 int64_t AmgDevice::device_bytes() const {
-  int64_t t = cinv.bytes() + lv.bytes();
+  int64_t t = cinv.bytes();
   for (int l = 0; l < nlev; ++l) {
     t += A[l].slice_ptr.bytes() + A[l].col.bytes() + P[l].slice_ptr.bytes() + P[l].col.bytes() + rrp[l].bytes() +
          rcol[l].bytes() + val[l].bytes() + pval[l].bytes() + rval[l].bytes() + dinv[l].bytes() + vec[l].bytes();
@@ -231,8 +238,11 @@ int64_t AmgDevice::device_bytes() const {
 // ------------------------------------------------------------------ device phases
 namespace {
 
+// 768 threads (80 registers): u1 of the 400x400x2 film / the 64 boxes / the 20x20x5 box 45.5 /
+// 34.2 / 6.9 ms per 40 solves; 1024 threads (64 registers, spills) 45.5 / 37.5 / 7.6, 512 threads
+// 48.1 / 34.9 / 6.8 (fewer rows in flight)
 #ifndef SPX_PCG_BLOCK
-#define SPX_PCG_BLOCK 1024
+#define SPX_PCG_BLOCK 768
 #endif
 #ifndef SPX_PCG_CTAS_PER_SM
 #define SPX_PCG_CTAS_PER_SM 1
@@ -287,48 +297,6 @@ __device__ __forceinline__ float4 ld_hint4(const float4* a, uint64_t pol) {
   return v;
 }
 
-__device__ __forceinline__ float ld_hint(const __half* a, uint64_t pol) {
-  unsigned short v;
-  asm("ld.global.nc.L2::cache_hint.b16 %0, [%1], %2;" : "=h"(v) : "l"(a), "l"(pol));
-  return __half2float(__ushort_as_half(v));
-}
-
-// row dot products of one SELL-32 slice (values and columns are read-only for the kernel's
-// lifetime; loaded with the L2 policy `pol`); VT = float or __half values
-template <class VT>
-__device__ __forceinline__ float sell_dot(const int64_t* __restrict__ sp, const int32_t* __restrict__ col,
-                                          const VT* __restrict__ val, int64_t sl, int lane,
-                                          const float* __restrict__ v, uint64_t pol) {
-  const int64_t base = sp[sl];
-  const int width = static_cast<int>((sp[sl + 1] - base) >> 5);
-  const VT* vv = val + base + lane;
-  const int32_t* cc = col + base + lane;
-  float a0 = 0.0f, a1 = 0.0f;
-  int k = 0;
-  for (; k + 8 <= width; k += 8) {  // eight gathers in flight per thread
-    float w[8];
-    int32_t c[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      w[u] = ld_hint(vv + (k + u) * 32, pol);
-      c[u] = ld_hint(cc + (k + u) * 32, pol);
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u += 2) {
-      a0 += w[u] * v[c[u]];
-      a1 += w[u + 1] * v[c[u + 1]];
-    }
-  }
-  for (; k + 2 <= width; k += 2) {
-    const float w0 = ld_hint(vv + k * 32, pol), w1 = ld_hint(vv + (k + 1) * 32, pol);
-    const int32_t c0 = ld_hint(cc + k * 32, pol), c1 = ld_hint(cc + (k + 1) * 32, pol);
-    a0 += w0 * v[c0];
-    a1 += w1 * v[c1];
-  }
-  if (k < width) a0 += ld_hint(vv + k * 32, pol) * v[ld_hint(cc + k * 32, pol)];
-  return a0 + a1;
-}
-
 // Slice bounds of SELL-32 slice sl (zero width past the last slice); the PCG product phase
 // loads the bounds of a warp's next slice while it works on the current one.
 __device__ __forceinline__ void slice_bounds(const int64_t* __restrict__ sp, int64_t sl, int64_t ns, int64_t& base,
@@ -339,135 +307,6 @@ __device__ __forceinline__ void slice_bounds(const int64_t* __restrict__ sp, int
   } else {
     base = 0;
     width = 0;
-  }
-}
-
-// level matrix times a level vector for one slice, with the FP16 sweep values when present
-__device__ __forceinline__ float lvl_dot(const AmgLevelDev& L, int64_t sl, int lane, const float* __restrict__ v) {
-  return L.val16 ? sell_dot(L.sp, L.col, L.val16, sl, lane, v, l2_policy_keep())
-                 : sell_dot(L.sp, L.col, L.val, sl, lane, v, l2_policy_keep());
-}
-
-// pre-smoothing from x = 0, Chebyshev steps 1 and 2 (one SpMV: A d0, d0 = D^-1 b / theta)
-__device__ void pre_a(const AmgLevelDev& L, RowRange rr) {
-  const float rho0 = 1.0f / L.sigma, rho1 = 1.0f / (2.0f * L.sigma - rho0);
-  for (int64_t sl = rr.gw; sl < L.nslices; sl += rr.nw) {
-    const int64_t i = sl * 32 + rr.lane;
-    const float t = lvl_dot(L, sl, rr.lane, L.db);
-    if (i < L.n) {
-      const float di = L.dinv[i];
-      const float d0 = L.db[i] / L.theta;
-      const float r1 = L.db[i] - di * t / L.theta;
-      const float d1 = rho1 * rho0 * d0 + (2.0f * rho1 / L.delta) * r1;
-      L.x[i] = d0 + d1;
-      L.d[i] = d1;
-      L.r[i] = r1;
-    }
-  }
-}
-
-// residual b - A x after pre-smoothing (A d1), stored in r
-__device__ void pre_b(const AmgLevelDev& L, RowRange rr) {
-  for (int64_t sl = rr.gw; sl < L.nslices; sl += rr.nw) {
-    const int64_t i = sl * 32 + rr.lane;
-    const float t = lvl_dot(L, sl, rr.lane, L.d);
-    if (i < L.n) {
-      const float di = L.dinv[i];
-      L.r[i] = (L.r[i] - di * t) / di;
-    }
-  }
-}
-
-// b_c = R r (CSR rows, `r_lanes` lanes per row), db_c = D_c^-1 b_c
-__device__ void restrict_to(const AmgLevelDev& L, const AmgLevelDev& C, RowRange rr) {
-  const int G = L.r_lanes;
-  const int gl = rr.lane & (G - 1);
-  const int64_t rows_per_warp = 32 / G;
-  const int64_t first = rr.gw * rows_per_warp + rr.lane / G, stride = rr.nw * rows_per_warp;
-  const int64_t nrows_pad = (C.n + rows_per_warp - 1) / rows_per_warp * rows_per_warp;
-  for (int64_t a = first - rr.lane / G; a < nrows_pad; a += stride) {  // uniform per warp
-    const int64_t row = a + rr.lane / G;
-    float t = 0.0f;
-    if (row < C.n) {
-      const int64_t k1 = L.r_rp[row + 1];
-      int64_t k = L.r_rp[row] + gl;
-      for (; k + 3 * G < k1; k += 4 * G) {  // four gathers in flight per lane
-        const float w0 = L.r_val[k], w1 = L.r_val[k + G], w2 = L.r_val[k + 2 * G], w3 = L.r_val[k + 3 * G];
-        const int32_t c0 = L.r_col[k], c1 = L.r_col[k + G], c2 = L.r_col[k + 2 * G], c3 = L.r_col[k + 3 * G];
-        t += w0 * L.r[c0] + w1 * L.r[c1] + w2 * L.r[c2] + w3 * L.r[c3];
-      }
-      for (; k < k1; k += G) t += L.r_val[k] * L.r[L.r_col[k]];
-    }
-    for (int o = G >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (row < C.n && gl == 0) {
-      C.b[row] = t;
-      C.db[row] = C.dinv[row] * t;
-    }
-  }
-}
-
-__device__ void prolong_from(const AmgLevelDev& L, const AmgLevelDev& C, RowRange rr) {
-  for (int64_t sl = rr.gw; sl < L.p_nslices; sl += rr.nw) {
-    const int64_t i = sl * 32 + rr.lane;
-    const float t = sell_dot(L.p_sp, L.p_col, L.p_val, sl, rr.lane, C.x, l2_policy_stream());
-    if (i < L.n) L.x[i] += t;
-  }
-}
-
-// post-smoothing from x, Chebyshev step 1 (r0 = D^-1 (b - A x), x2 = x + r0 / theta)
-__device__ void post_c(const AmgLevelDev& L, RowRange rr) {
-  for (int64_t sl = rr.gw; sl < L.nslices; sl += rr.nw) {
-    const int64_t i = sl * 32 + rr.lane;
-    const float t = lvl_dot(L, sl, rr.lane, L.x);
-    if (i < L.n) {
-      const float r0 = L.db[i] - L.dinv[i] * t;
-      const float d0 = r0 / L.theta;
-      L.x2[i] = L.x[i] + d0;
-      L.d[i] = d0;
-      L.r[i] = r0;
-    }
-  }
-}
-
-// post-smoothing step 2; on the top level also the partial dots (r64, z^), (w, z^) of the PCG
-__device__ void post_d(const AmgLevelDev& L, RowRange rr, const double* __restrict__ r64,
-                       const double* __restrict__ sdinv, double& rz, double& wz, bool top) {
-  const float rho0 = 1.0f / L.sigma, rho1 = 1.0f / (2.0f * L.sigma - rho0);
-  for (int64_t sl = rr.gw; sl < L.nslices; sl += rr.nw) {
-    const int64_t i = sl * 32 + rr.lane;
-    const float t = lvl_dot(L, sl, rr.lane, L.d);
-    if (i < L.n) {
-      const float r1 = L.r[i] - L.dinv[i] * t;
-      const float d1 = rho1 * rho0 * L.d[i] + (2.0f * rho1 / L.delta) * r1;
-      const float z = L.x2[i] + d1;
-      L.x[i] = z;
-      if (top) {  // level 0 runs unscaled: z is u = D^-1/2 z^, z^ = u / sdinv
-        const double zh = static_cast<double>(z) / sdinv[i];
-        rz += r64[i] * zh;
-        wz += zh / sdinv[i];
-      }
-    }
-  }
-}
-
-// x = C^-1 b on the dense coarsest level: a warp per row over the grid, 16-byte loads of the
-// zero-padded rows (ld = nc rounded up to 4; b is read up to ld, inside the level's vectors)
-__device__ void coarse_solve(const AmgLevelDev& L, const float* __restrict__ cinv, int64_t nc, int64_t ldc,
-                             RowRange rr) {
-  const int64_t nv = ldc / 4;
-  const uint64_t pol = l2_policy_keep();  // the inverse stays in L2 across iterations
-  const float4* b4 = reinterpret_cast<const float4*>(L.b);
-  for (int64_t i = rr.gw; i < nc; i += rr.nw) {
-    const float4* row = reinterpret_cast<const float4*>(cinv + i * ldc);
-    float s = 0.0f;
-#pragma unroll 4
-    for (int64_t j = rr.lane; j < nv; j += 32) {
-      const float4 c = ld_hint4(row + j, pol);
-      const float4 b = b4[j];
-      s += c.x * b.x + c.y * b.y + c.z * b.z + c.w * b.w;
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (rr.lane == 0) L.x[i] = s;
   }
 }
 
@@ -694,11 +533,11 @@ __device__ void post_c_r(const AmgLevelDev& L, RowRange rr) {
   }
 }
 
-// on the top level also the partial dots (r64, z^), (w, z^) over all R blocks; r64 is the
-// interleaved PCG residual, sdinv the block-ordered (replicated) scaling
+// on the top level also the partial dots (r64, u), (d, u) over all R blocks; r64 is the
+// interleaved PCG residual, diag the (replicated) diagonal
 template <int R>
 __device__ void post_d_r(const AmgLevelDev& L, RowRange rr, const double* __restrict__ r64,
-                         const double* __restrict__ sdinv, double& rz, double& wz, bool top) {
+                         const double* __restrict__ diag, double& rz, double& wz, bool top) {
   const float rho0 = 1.0f / L.sigma, rho1 = 1.0f / (2.0f * L.sigma - rho0);
   for (int64_t sl = rr.gw; sl < L.nslices; sl += rr.nw) {
     const int64_t i = sl * 32 + rr.lane;
@@ -706,7 +545,7 @@ __device__ void post_d_r(const AmgLevelDev& L, RowRange rr, const double* __rest
     sell_dot_r<R>(L.sp, L.col, L.val, sl, rr.lane, L.d, l2_policy_keep(), t);
     if (i < L.n) {
       const float di = L.dinv[i];
-      const double sd = top ? sdinv[i] : 1.0;
+      const double dg = top ? diag[i] : 0.0;
       float rv[R], dv[R], x2[R], zo[R];
       load_r<R>(L.r, i, rv);
       load_r<R>(L.d, i, dv);
@@ -718,9 +557,8 @@ __device__ void post_d_r(const AmgLevelDev& L, RowRange rr, const double* __rest
         const float z = x2[r] + d1;
         zo[r] = z;
         if (top) {
-          const double zh = static_cast<double>(z) / sd;
-          rz += r64[i * R + r] * zh;
-          wz += zh / sd;
+          rz += r64[i * R + r] * static_cast<double>(z);
+          wz += dg * static_cast<double>(z);
         }
       }
       store_r<R>(L.x, i, zo);
@@ -770,10 +608,9 @@ struct PcgParams {
   int64_t n, nslices;
   const int64_t* sp;
   const int32_t* col;
-  const double* v64;   // scaled FP64 values (true residual)
-  const float* a32;    // unscaled FP32 values (difference-form SpMV)
-  const double* rsum;  // row sums of the unscaled matrix
-  const double* sdinv;
+  const double* a64;   // FP64 values (true residual)
+  const float* a32;    // FP32 values (difference-form SpMV)
+  const double* rsum;  // row sums of the matrix
   const double* diag;
   const TV* b;
   TV* x;
@@ -787,13 +624,14 @@ struct PcgParams {
   double* res_acc;
   double rtol, atol, ww;
   int maxit, max_outer, warm, project;
-  int bh_given;  // bh already holds the scaled, projected right-hand side (FP64)
-  const AmgLevelDev* lv;
+  int bh_given;  // bh already holds the projected right-hand side (FP64)
   int nlev;
   const float* cinv;
   int64_t nc, ldc;
   int reps;  // identical blocks: vectors hold reps x n entries, the matrix n rows
   int timing;  // phase timing marks on (spx_debug_pcg_timing)
+  AmgLevelDev L[AMG_MAX_LEVELS];
+  AmgResident R[AMG_MAX_LEVELS];
 };
 
 #define PCG_ROWS_BEGIN                                              \
@@ -842,206 +680,539 @@ __device__ __forceinline__ void pcg_mark(unsigned long long& t_prev, int slot, i
   }
 }
 
-// z^ = V(r^): lv[0].b / lv[0].db hold the unscaled residual D^1/2 r^ (FP32) on entry, lv[0].x
-// holds u = D^-1/2 z^ on exit, and slot `slot` of the partials holds (r^, z^), (w, z^).  nlev >= 2.
+// ---- one system (k_pcg_amg): CTA-owned blocks of slices, kept in shared memory
+extern __shared__ __align__(16) int32_t pcg_words[];
+constexpr int PCG_DYN_MAX = 220 * 1024;  // dynamic shared memory; the rest is for static data and L1
+
+// this CTA's block of one level: slices [s0, s0 + cnt), the first nres of them resident
+struct LvlBlock {
+  int64_t s0;
+  int64_t base, pbase;  // first entries of the block's rows of A and P in global memory
+  int64_t r0, rbase;  // coarse rows [r0, r0 + rcnt) of the restriction, their first entry
+  int32_t cnt, nres, rcnt;
+};
+struct PcgShared {
+  LvlBlock blk[AMG_MAX_LEVELS];
+  double red[64], tot[2];
+  int ok;
+};
+
+// bounds of slice k of the block, relative to its first entry
+__device__ __forceinline__ void block_bounds(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B, int k,
+                                             int64_t& o, int& width) {
+  if (R.off >= 0) {
+    const int32_t a = pcg_words[R.off + k], e = pcg_words[R.off + k + 1];
+    o = a;
+    width = (e - a) >> 5;
+  } else {
+    const int64_t a = L.sp[B.s0 + k];
+    o = a - B.base;
+    width = static_cast<int>((L.sp[B.s0 + k + 1] - a) >> 5);
+  }
+}
+
+// sum_k w_k f(v[c_k]) over the entries of one row: eight gathers in flight; entries from shared
+// memory (resident slice) or through L2.  f is applied to the gathered value.
+template <class TA, class F>
+__device__ __forceinline__ TA block_dot(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B, int k, int lane,
+                                        const float* v, F f) {
+  int64_t o;
+  int width;
+  block_bounds(L, R, B, k, o, width);
+  TA a0 = TA(0), a1 = TA(0);
+  if (k < B.nres) {
+    const int wv = R.val + static_cast<int>(o) + lane, wc = R.col + static_cast<int>(o) + lane;
+    for (int j = 0; j < width; j += 8) {
+      float g[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) g[u] = j + u < width ? v[pcg_words[wc + (j + u) * 32]] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        if (j + u < width) a0 += static_cast<TA>(__int_as_float(pcg_words[wv + (j + u) * 32])) * f(g[u]);
+        if (j + u + 1 < width) a1 += static_cast<TA>(__int_as_float(pcg_words[wv + (j + u + 1) * 32])) * f(g[u + 1]);
+      }
+    }
+  } else {
+    const uint64_t pol = l2_policy_keep();
+    const float* gv = L.val + B.base + o + lane;
+    const int32_t* gc = L.col + B.base + o + lane;
+    for (int j = 0; j < width; j += 8) {
+      int32_t c[8];
+      float w[8], g[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const bool in = j + u < width;
+        c[u] = in ? ld_hint(gc + (j + u) * 32, pol) : 0;
+        w[u] = in ? ld_hint(gv + (j + u) * 32, pol) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) g[u] = j + u < width ? v[c[u]] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        if (j + u < width) a0 += static_cast<TA>(w[u]) * f(g[u]);
+        if (j + u + 1 < width) a1 += static_cast<TA>(w[u + 1]) * f(g[u + 1]);
+      }
+    }
+  }
+  return a0 + a1;
+}
+__device__ __forceinline__ float block_dot(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B, int k,
+                                           int lane, const float* v) {
+  return block_dot<float>(L, R, B, k, lane, v, [](float g) { return g; });
+}
+
+// rows of this CTA's block of a level; the body sees k (slice of the block) and i (row)
+#define BLOCK_ROWS_BEGIN(B, nrows)                                              \
+  for (int k = threadIdx.x >> 5; k < (B).cnt; k += blockDim.x >> 5) {           \
+    const int lane = threadIdx.x & 31;                                          \
+    const int64_t i = ((B).s0 + k) * 32 + lane;                                 \
+    if (i < (nrows)) {
+#define BLOCK_ROWS_END \
+  }                    \
+  }
+
+// pre-smoothing from x = 0, Chebyshev steps 1 and 2 (one SpMV: A d0, d0 = D^-1 b / theta)
+__device__ __forceinline__ void pre_a(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B) {
+  const float rho0 = 1.0f / L.sigma, rho1 = 1.0f / (2.0f * L.sigma - rho0);
+  const float it = 1.0f / L.theta, c0 = rho1 * rho0, c1 = 2.0f * rho1 / L.delta;
+  BLOCK_ROWS_BEGIN(B, L.n)
+    const float di = L.dinv[i], db = L.db[i];
+    const float t = block_dot(L, R, B, k, lane, L.db);
+    const float d0 = db * it;
+    const float r1 = db - di * t * it;
+    const float d1 = c0 * d0 + c1 * r1;
+    L.x[i] = d0 + d1;
+    L.d[i] = d1;
+    L.r[i] = r1;
+  BLOCK_ROWS_END
+}
+
+// residual b - A x after pre-smoothing (A d1), stored in r
+__device__ __forceinline__ void pre_b(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B) {
+  BLOCK_ROWS_BEGIN(B, L.n)
+    const float di = L.dinv[i], r = L.r[i];
+    const float t = block_dot(L, R, B, k, lane, L.d);
+    L.r[i] = r / di - t;
+  BLOCK_ROWS_END
+}
+
+// b_c = R r (CSR rows, `r_lanes` lanes per row), db_c = D_c^-1 b_c; each CTA takes a contiguous
+// block of the coarse rows, whose bounds it keeps in shared memory
+__device__ __forceinline__ void restrict_to(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B,
+                                            const AmgLevelDev& C) {
+  const int lane = threadIdx.x & 31, G = L.r_lanes, gl = lane & (G - 1), rpw = 32 / G;
+  for (int a = (threadIdx.x >> 5) * rpw; a < B.rcnt; a += (blockDim.x >> 5) * rpw) {  // uniform per warp
+    const int q = a + lane / G;
+    const int64_t row = B.r0 + q;
+    float t = 0.0f, di = 0.0f;
+    if (q < B.rcnt) {
+      int64_t k, k1;
+      if (R.off >= 0) {
+        k = B.rbase + pcg_words[R.roff + q] + gl;
+        k1 = B.rbase + pcg_words[R.roff + q + 1];
+      } else {
+        k = L.r_rp[row] + gl;
+        k1 = L.r_rp[row + 1];
+      }
+      di = C.dinv[row];
+      for (; k < k1; k += 8 * G) {  // eight gathers in flight per lane
+        int32_t c[8];
+        float w[8], g[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool in = k + u * G < k1;
+          c[u] = in ? L.r_col[k + u * G] : 0;
+          w[u] = in ? L.r_val[k + u * G] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) g[u] = k + u * G < k1 ? L.r[c[u]] : 0.0f;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t += w[u] * g[u];
+      }
+    }
+    for (int o = G >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (q < B.rcnt && gl == 0) {
+      C.b[row] = t;
+      C.db[row] = di * t;
+    }
+  }
+}
+
+// x += P x_c; P has the rows of L and so its slices (L's block)
+__device__ __forceinline__ void prolong_from(const AmgLevelDev& L, const AmgResident& R, const AmgLevelDev& C,
+                                             const LvlBlock& B) {
+  BLOCK_ROWS_BEGIN(B, L.n)
+    int64_t base;
+    int width;
+    if (R.off >= 0) {
+      const int32_t o = pcg_words[R.poff + k];
+      base = B.pbase + o;
+      width = (pcg_words[R.poff + k + 1] - o) >> 5;
+    } else {
+      base = L.p_sp[B.s0 + k];
+      width = static_cast<int>((L.p_sp[B.s0 + k + 1] - base) >> 5);
+    }
+    const float xi = L.x[i];
+    const float* pv = L.p_val + base + lane;
+    const int32_t* pc = L.p_col + base + lane;
+    float t = 0.0f;
+    for (int j = 0; j < width; j += 4) {
+      int32_t c[4];
+      float w[4], g[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = j + u < width;
+        c[u] = in ? pc[(j + u) * 32] : 0;
+        w[u] = in ? pv[(j + u) * 32] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) g[u] = j + u < width ? C.x[c[u]] : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) t += w[u] * g[u];
+    }
+    L.x[i] = xi + t;
+  BLOCK_ROWS_END
+}
+
+// post-smoothing from x, Chebyshev step 1 (r0 = D^-1 (b - A x), x2 = x + r0 / theta)
+__device__ __forceinline__ void post_c(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B) {
+  const float it = 1.0f / L.theta;
+  BLOCK_ROWS_BEGIN(B, L.n)
+    const float di = L.dinv[i], db = L.db[i], x = L.x[i];
+    const float t = block_dot(L, R, B, k, lane, L.x);
+    const float r0 = db - di * t;
+    L.x2[i] = x + r0 * it;
+    L.r[i] = r0;
+  BLOCK_ROWS_END
+}
+
+// post-smoothing step 2 (d0 = r0 / theta); on the top level also the partial dots (r64, u) and
+// (d, u) of the PCG
+template <bool TOP>
+__device__ __forceinline__ void post_d(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B, const double* r64,
+                                       double& rz, double& wz) {
+  const float rho0 = 1.0f / L.sigma, rho1 = 1.0f / (2.0f * L.sigma - rho0);
+  const float it = 1.0f / L.theta, c0 = rho1 * rho0 * it, c1 = 2.0f * rho1 / L.delta;
+  BLOCK_ROWS_BEGIN(B, L.n)
+    const float di = L.dinv[i], r0 = L.r[i], x2 = L.x2[i];
+    const double rd = TOP ? r64[i] : 0.0;
+    const float t = block_dot(L, R, B, k, lane, L.r) * it;
+    const float r1 = r0 - di * t;
+    const float z = x2 + (c0 * r0 + c1 * r1);
+    L.x[i] = z;
+    if (TOP) {
+      rz += rd * static_cast<double>(z);
+      wz += static_cast<double>(z / di);
+    }
+  BLOCK_ROWS_END
+}
+
+// x = C^-1 b on the dense coarsest level: each CTA takes a contiguous block of rows, its warps
+// split evenly over them (several warps to a row on the few rows of a CTA, their sums joined in
+// shared memory); 16-byte loads of the zero-padded rows (ld = nc rounded up to 4; b is read up
+// to ld, inside the level's vectors), nine of a lane in flight.
+__device__ __forceinline__ void coarse_solve(const AmgLevelDev& L, const float* __restrict__ cinv, int64_t nc,
+                                             int64_t ldc, double* red) {
+  const int nv = static_cast<int>(ldc / 4), warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r0 = static_cast<int>(nc * blockIdx.x / gridDim.x), r1 = static_cast<int>(nc * (blockIdx.x + 1) / gridDim.x);
+  const uint64_t pol = l2_policy_keep();  // the inverse stays in L2 across iterations
+  const float4* b4 = reinterpret_cast<const float4*>(L.b);
+  float* fr = reinterpret_cast<float*>(red);
+  int wpr = 1;  // warps per row
+  while (wpr * 2 * (r1 - r0) <= warps && wpr < 32) wpr *= 2;
+  const int rows = warps / wpr, part = warp & (wpr - 1);
+  for (int a = r0; a < r1; a += rows) {  // uniform per CTA
+    const int i = a + warp / wpr;
+    float s = 0.0f;
+    if (i < r1) {
+      const float4* row = reinterpret_cast<const float4*>(cinv + static_cast<int64_t>(i) * ldc);
+#pragma unroll 9
+      for (int j = part * 32 + lane; j < nv; j += 32 * wpr) {
+        const float4 c = ld_hint4(row + j, pol);
+        const float4 b = b4[j];
+        s += c.x * b.x + c.y * b.y + c.z * b.z + c.w * b.w;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (wpr == 1) {
+      if (lane == 0 && i < r1) L.x[i] = s;
+    } else {
+      if (lane == 0) fr[warp] = s;
+      __syncthreads();
+      if (part == 0 && lane == 0 && i < r1) {
+        for (int q = 1; q < wpr; ++q) s += fr[warp + q];
+        L.x[i] = s;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Grid barrier with two sums: every CTA's partials of a and b are written before its arrival and
+// added up, in the same order in every CTA, by the waiting warp before it releases its CTA.
+// `flip` alternates the two slots of the partials: a CTA writes a slot again only after the
+// barrier that follows every CTA's last read of it.  Bounded wait as in grid_barrier.
 template <class TV>
-__device__ bool vcycle(const PcgParams<TV>& P, int slot, double* sh, unsigned long long& tm) {
+__device__ __forceinline__ bool sync_sum(const PcgParams<TV>& P, PcgShared& S, int& flip, double& a, double& b) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nb = gridDim.x;
+  a = warp_sum(a);
+  b = warp_sum(b);
+  if (lane == 0) {
+    S.red[2 * wid] = a;
+    S.red[2 * wid + 1] = b;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    const int nw = blockDim.x >> 5;
+    double u = warp_sum(lane < nw ? S.red[2 * lane] : 0.0);
+    double v = warp_sum(lane < nw ? S.red[2 * lane + 1] : 0.0);
+    double* part = P.part + static_cast<int64_t>(flip) * 2 * nb;
+    int ok = 1;
+    if (lane == 0) {
+      part[2 * blockIdx.x] = u;
+      part[2 * blockIdx.x + 1] = v;
+      ok = grid_arrive_wait(P.bar, nb, P.err) ? 1 : 0;
+      S.ok = ok;
+    }
+    __syncwarp();
+    u = v = 0.0;
+    for (int c = lane; c < nb; c += 32) {
+      const double2 q = __ldcg(reinterpret_cast<const double2*>(part) + c);
+      u += q.x;
+      v += q.y;
+    }
+    u = warp_sum(u);
+    v = warp_sum(v);
+    if (lane == 0) {
+      S.tot[0] = u;
+      S.tot[1] = v;
+    }
+  }
+  flip ^= 1;
+  __syncthreads();
+  a = S.tot[0];
+  b = S.tot[1];
+  return S.ok != 0;
+}
+
+// u = V(r): L[0].db holds D^-1 r (FP32) on entry, L[0].x holds u on exit; rz, wz: (r, u), (d, u)
+// over the grid.  nlev >= 2.
+template <class TV>
+__device__ __forceinline__ bool vcycle(const PcgParams<TV>& P, PcgShared& S, int& flip, double& rz, double& wz,
+                                       unsigned long long& tm) {
   const unsigned nb = gridDim.x;
   unsigned int* cnt = P.bar;
-  unsigned int* gen = P.bar + 1;
-  const RowRange rr{static_cast<int64_t>((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5),
-                    static_cast<int64_t>((gridDim.x * static_cast<int64_t>(blockDim.x)) >> 5),
-                    static_cast<int>(threadIdx.x & 31)};
   const int NL = P.nlev;
   int ph = 0;
   for (int l = 0; l + 1 < NL; ++l) {
-    const AmgLevelDev& L = P.lv[l];
-    pre_a(L, rr);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+    const AmgLevelDev& L = P.L[l];
+    pre_a(L, P.R[l], S.blk[l]);
+    if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
-    pre_b(L, rr);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+    pre_b(L, P.R[l], S.blk[l]);
+    if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
-    restrict_to(L, P.lv[l + 1], rr);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+    restrict_to(L, P.R[l], S.blk[l], P.L[l + 1]);
+    if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
   }
-  coarse_solve(P.lv[NL - 1], P.cinv, P.nc, P.ldc, rr);
-  if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+  coarse_solve(P.L[NL - 1], P.cinv, P.nc, P.ldc, S.red);
+  if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
   pcg_mark(tm, ph++, P.timing);
+  rz = wz = 0.0;
   for (int l = NL - 2; l >= 0; --l) {
-    const AmgLevelDev& L = P.lv[l];
-    prolong_from(L, P.lv[l + 1], rr);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+    const AmgLevelDev& L = P.L[l];
+    prolong_from(L, P.R[l], P.L[l + 1], S.blk[l]);
+    if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
-    post_c(L, rr);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+    post_c(L, P.R[l], S.blk[l]);
+    if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
-    double rz = 0.0, wz = 0.0;
-    post_d(L, rr, P.r, P.sdinv, rz, wz, l == 0);
-    if (l == 0) cta_partial(P.part, slot, rz, wz, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return false;
+    if (l == 0) {
+      post_d<true>(L, P.R[l], S.blk[l], P.r, rz, wz);
+      if (!sync_sum(P, S, flip, rz, wz)) return false;
+    } else {
+      post_d<false>(L, P.R[l], S.blk[l], nullptr, rz, wz);
+      if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
+    }
     pcg_mark(tm, ph++, P.timing);
   }
   return true;
 }
 
 template <class TV>
-__global__ void __launch_bounds__(PCG_BLOCK, PCG_CTAS_PER_SM) k_pcg_amg(PcgParams<TV> P) {
+__global__ void __launch_bounds__(PCG_BLOCK, PCG_CTAS_PER_SM) k_pcg_amg(const __grid_constant__ PcgParams<TV> P) {
   unsigned long long tm = 0ull;
-  __shared__ double sh[160];
-  const unsigned nb = gridDim.x;
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
-  unsigned int* cnt = P.bar;
-  unsigned int* gen = P.bar + 1;
+  __shared__ PcgShared S;
+  int flip = 0;
   const int64_t n = P.n;
-  float* b0 = P.lv[0].b;
-  float* db0 = P.lv[0].db;
-  const float* dinv0 = P.lv[0].dinv;
-  double tot[4];
-  double meanb = 0.0;
+  // this CTA's blocks: bounds, how much of each is resident, the resident entries
+  for (int l = threadIdx.x; l + 1 < P.nlev; l += blockDim.x) {
+    LvlBlock B;
+    B.s0 = P.L[l].nslices * blockIdx.x / gridDim.x;
+    B.cnt = static_cast<int32_t>(P.L[l].nslices * (blockIdx.x + 1) / gridDim.x - B.s0);
+    B.base = P.L[l].sp[B.s0];
+    B.pbase = P.L[l].p_sp[B.s0];
+    B.nres = 0;
+    const int64_t ncr = P.L[l + 1].n;
+    B.r0 = ncr * blockIdx.x / gridDim.x;
+    B.rcnt = static_cast<int32_t>(ncr * (blockIdx.x + 1) / gridDim.x - B.r0);
+    B.rbase = P.L[l].r_rp[B.r0];
+    S.blk[l] = B;
+  }
+  __syncthreads();
+  for (int l = 0; l + 1 < P.nlev; ++l) {
+    const LvlBlock& B = S.blk[l];
+    if (P.R[l].off >= 0)
+      for (int k = threadIdx.x; k <= B.cnt; k += blockDim.x) {
+        pcg_words[P.R[l].off + k] = static_cast<int32_t>(P.L[l].sp[B.s0 + k] - B.base);
+        pcg_words[P.R[l].poff + k] = static_cast<int32_t>(P.L[l].p_sp[B.s0 + k] - B.pbase);
+      }
+    if (P.R[l].off >= 0)
+      for (int k = threadIdx.x; k <= B.rcnt; k += blockDim.x)
+        pcg_words[P.R[l].roff + k] = static_cast<int32_t>(P.L[l].r_rp[B.r0 + k] - B.rbase);
+  }
+  __syncthreads();
+  if (threadIdx.x < P.nlev - 1 && P.R[threadIdx.x].off >= 0) {  // last slice bound within the capacity
+    const int l = threadIdx.x;
+    int lo = 0, hi = S.blk[l].cnt;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (pcg_words[P.R[l].off + mid] <= P.R[l].cap) lo = mid; else hi = mid - 1;
+    }
+    S.blk[l].nres = lo;
+  }
+  __syncthreads();
+  for (int l = 0; l + 1 < P.nlev; ++l) {
+    const LvlBlock& B = S.blk[l];
+    if (B.nres == 0) continue;
+    const int m4 = pcg_words[P.R[l].off + B.nres] / 4;  // whole 32-entry columns
+    const float4* gv = reinterpret_cast<const float4*>(P.L[l].val + B.base);
+    const int4* gc = reinterpret_cast<const int4*>(P.L[l].col + B.base);
+    float4* sv = reinterpret_cast<float4*>(pcg_words + P.R[l].val);
+    int4* sc = reinterpret_cast<int4*>(pcg_words + P.R[l].col);
+    for (int k = threadIdx.x; k < m4; k += blockDim.x) {
+      sv[k] = gv[k];
+      sc[k] = gc[k];
+    }
+  }
+  __syncthreads();
+  const LvlBlock B0 = S.blk[0];
+  const AmgLevelDev& L0 = P.L[0];
+  double meanb = 0.0, dummy = 0.0;
   if (P.project && !P.bh_given) {
     double part = 0.0;
-    PCG_ROWS_BEGIN part += static_cast<double>(P.b[row]);
-    PCG_ROWS_END
-    cta_partial(P.part, 0, part, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    cta_total(P.part, 0, tot, sh);
-    meanb = tot[0] / static_cast<double>(n);
+    BLOCK_ROWS_BEGIN(B0, n) part += static_cast<double>(P.b[i]);
+    BLOCK_ROWS_END
+    if (!sync_sum(P, S, flip, part, dummy)) return;
+    meanb = part / static_cast<double>(n);
   }
-  {
-    double bb = 0.0;
-    PCG_ROWS_BEGIN
-      double bv;
-      if (P.bh_given) {
-        bv = P.bh[row] / P.sdinv[row];
-      } else {
-        bv = static_cast<double>(P.b[row]) - meanb;
-        P.bh[row] = bv * P.sdinv[row];
-      }
-      if (!P.warm) P.y[row] = 0.0;
-      bb += bv * bv;
-    PCG_ROWS_END
-    cta_partial(P.part, 1, bb, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  cta_total(P.part, 1, tot, sh);
-  const double bb = tot[0];
+  double bb = 0.0;
+  BLOCK_ROWS_BEGIN(B0, n)
+    double bv;
+    if (P.bh_given) {
+      bv = P.bh[i];
+    } else {
+      bv = static_cast<double>(P.b[i]) - meanb;
+      P.bh[i] = bv;
+    }
+    if (!P.warm) P.y[i] = 0.0;
+    bb += bv * bv;
+  BLOCK_ROWS_END
+  dummy = 0.0;
+  if (!sync_sum(P, S, flip, bb, dummy)) return;
   if (P.warm && !(bb > 0.0)) {  // b = 0: the solution is 0
-    PCG_ROWS_BEGIN P.y[row] = 0.0;
-    PCG_ROWS_END
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
+    BLOCK_ROWS_BEGIN(B0, n) P.y[i] = 0.0;
+    BLOCK_ROWS_END
+    if (!grid_barrier(P.bar, nullptr, gridDim.x, P.err)) return;
   }
   const double tol2 = fmax(P.rtol * P.rtol * bb, P.atol * P.atol);
   int total = 0, outers = 0;
   double rr = 0.0, rr0 = -1.0;
   for (int outer = 0; outer < P.max_outer; ++outer) {
     ++outers;
-    // true residual r = bh - A^ y (FP64), its unscaled norm, r -> level-0 right-hand side
+    // true residual r = bh - A y (FP64), its norm, D^-1 r -> level-0 right-hand side
     {
       double rh = 0.0;
-      PCG_ROWS_BEGIN
+      const uint64_t pst = l2_policy_stream();
+      BLOCK_ROWS_BEGIN(B0, n)
+        int64_t o;
+        int width;
+        block_bounds(L0, P.R[0], B0, k, o, width);
+        const double bv = P.bh[i];
+        const float di = L0.dinv[i];
+        const double* gv = P.a64 + B0.base + o + lane;
+        const int32_t* gc = P.col + B0.base + o + lane;
+        const bool res = k < B0.nres;
+        const int wc = P.R[0].col + static_cast<int>(res ? o : 0) + lane;
         double acc = 0.0, acc2 = 0.0;
-        const uint64_t pst = l2_policy_stream(), pkeep = l2_policy_keep();
-        int k = 0;
-        for (; k + 2 <= width; k += 2) {
-          const int64_t idx = base + ((int64_t)k << 5) + lane;
-          acc += ld_hint(P.v64 + idx, pst) * P.y[ld_hint(P.col + idx, pkeep)];
-          acc2 += ld_hint(P.v64 + idx + 32, pst) * P.y[ld_hint(P.col + idx + 32, pkeep)];
+        for (int j = 0; j < width; j += 4) {
+          double w[4], g[4];
+          int32_t c[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const bool in = j + u < width;
+            c[u] = in ? (res ? pcg_words[wc + (j + u) * 32] : gc[(j + u) * 32]) : 0;
+            w[u] = in ? ld_hint(gv + (j + u) * 32, pst) : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) g[u] = j + u < width ? P.y[c[u]] : 0.0;
+#pragma unroll
+          for (int u = 0; u < 4; u += 2) {
+            acc += w[u] * g[u];
+            acc2 += w[u + 1] * g[u + 1];
+          }
         }
-        if (k < width) {
-          const int64_t idx = base + ((int64_t)k << 5) + lane;
-          acc += ld_hint(P.v64 + idx, pst) * P.y[ld_hint(P.col + idx, pkeep)];
-        }
-        const double r = P.bh[row] - (acc + acc2);
-        P.r[row] = r;
-        const float rf = static_cast<float>(r / P.sdinv[row]);
-        b0[row] = rf;
-        db0[row] = dinv0[row] * rf;
-        rh += P.diag[row] * r * r;
-      PCG_ROWS_END
-      cta_partial(P.part, 0, rh, 0.0, 0.0, 0.0, sh);
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
+        const double r = bv - (acc + acc2);
+        P.r[i] = r;
+        L0.db[i] = di * static_cast<float>(r);
+        rh += r * r;
+      BLOCK_ROWS_END
+      dummy = 0.0;
+      if (!sync_sum(P, S, flip, rh, dummy)) return;
       pcg_mark(tm, 30, P.timing);
+      rr = rh;
     }
-    cta_total(P.part, 0, tot, sh);
-    rr = tot[0];
     if (rr0 < 0.0) rr0 = rr;
     if (rr <= tol2 || total >= P.maxit) break;
     double rz_old = 1.0;
     for (int it = 0;; ++it) {
-      if (!vcycle(P, 2, sh, tm)) return;
-      cta_total(P.part, 2, tot, sh);
-      const double rz = tot[0];
-      const double c = P.project && P.ww > 0.0 ? tot[1] / P.ww : 0.0;
+      double rz, wz;
+      if (!vcycle(P, S, flip, rz, wz, tm)) return;
+      const double c = P.project && P.ww > 0.0 ? wz / P.ww : 0.0;
       const double beta = it == 0 ? 0.0 : rz / rz_old;
-      const float* u0 = P.lv[0].x;  // u = D^-1/2 z^ from the unscaled level-0 cycle
+      const float* u0 = L0.x;  // u from the level-0 cycle
       double pq = 0.0;
-      PCG_SLICES_BEGIN
-        const double ui = static_cast<double>(u0[row]);
-        const uint64_t pkeep = l2_policy_keep();
-        double acc = 0.0, acc2 = 0.0;
-        int k = 0;
-        for (; k + 4 <= width; k += 4) {
-          const int64_t i0 = base + ((int64_t)k << 5) + lane;
-          const float w0 = ld_hint(P.a32 + i0, pkeep), w1 = ld_hint(P.a32 + i0 + 32, pkeep),
-                      w2 = ld_hint(P.a32 + i0 + 64, pkeep), w3 = ld_hint(P.a32 + i0 + 96, pkeep);
-          const int32_t c0 = ld_hint(P.col + i0, pkeep), c1 = ld_hint(P.col + i0 + 32, pkeep),
-                        c2 = ld_hint(P.col + i0 + 64, pkeep), c3 = ld_hint(P.col + i0 + 96, pkeep);
-          acc += static_cast<double>(w0) * (static_cast<double>(u0[c0]) - ui);
-          acc2 += static_cast<double>(w1) * (static_cast<double>(u0[c1]) - ui);
-          acc += static_cast<double>(w2) * (static_cast<double>(u0[c2]) - ui);
-          acc2 += static_cast<double>(w3) * (static_cast<double>(u0[c3]) - ui);
-        }
-        if (k < width) {  // up to three remaining columns, loaded together, summed in order
-          float wt[3];
-          int32_t ct[3];
-#pragma unroll
-          for (int u = 0; u < 3; ++u) {
-            const int64_t idx = base + ((int64_t)(k + u) << 5) + lane;
-            const bool in = k + u < width;
-            wt[u] = in ? ld_hint(P.a32 + idx, pkeep) : 0.0f;
-            ct[u] = in ? ld_hint(P.col + idx, pkeep) : 0;
-          }
-#pragma unroll
-          for (int u = 0; u < 3; ++u)
-            if (k + u < width) acc += static_cast<double>(wt[u]) * (static_cast<double>(u0[ct[u]]) - ui);
-        }
-        const double rsi = P.rsum[row], sdi = P.sdinv[row];
-        const double pold = it == 0 ? 0.0 : P.p[row], qold = it == 0 ? 0.0 : P.q[row];
-        acc = (acc + acc2 + rsi * ui) * sdi;
-        const double z = ui / sdi;
-        const double w = 1.0 / sdi;
-        const double pv = (z - c * w) + (it == 0 ? 0.0 : beta * pold);
-        const double qv = acc + (it == 0 ? 0.0 : beta * qold);
-        P.p[row] = pv;
-        P.q[row] = qv;
+      BLOCK_ROWS_BEGIN(B0, n)
+        const double ui = static_cast<double>(u0[i]), rsi = P.rsum[i];
+        const double pold = it == 0 ? 0.0 : P.p[i], qold = it == 0 ? 0.0 : P.q[i];
+        const double acc = block_dot<double>(L0, P.R[0], B0, k, lane, u0,
+                                             [ui](float g) { return static_cast<double>(g) - ui; });
+        const double pv = (ui - c) + (it == 0 ? 0.0 : beta * pold);
+        const double qv = (acc + rsi * ui) + (it == 0 ? 0.0 : beta * qold);
+        P.p[i] = pv;
+        P.q[i] = qv;
         pq += pv * qv;
-      PCG_SLICES_END
-      cta_partial(P.part, 3, pq, 0.0, 0.0, 0.0, sh);
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
+      BLOCK_ROWS_END
+      dummy = 0.0;
+      if (!sync_sum(P, S, flip, pq, dummy)) return;
       pcg_mark(tm, 28, P.timing);
-      cta_total(P.part, 3, tot, sh);
-      const double pqt = tot[0];
-      if (!(pqt > 0.0) || !(rz > 0.0)) break;
-      const double alpha = rz / pqt;
+      if (!(pq > 0.0) || !(rz > 0.0)) break;
+      const double alpha = rz / pq;
       double rh = 0.0;
-      PCG_ROWS_BEGIN
-        P.y[row] += alpha * P.p[row];
-        const double r = P.r[row] - alpha * P.q[row];
-        P.r[row] = r;
-        const float rf = static_cast<float>(r / P.sdinv[row]);
-        b0[row] = rf;
-        db0[row] = dinv0[row] * rf;
-        rh += P.diag[row] * r * r;
-      PCG_ROWS_END
-      cta_partial(P.part, 0, rh, 0.0, 0.0, 0.0, sh);
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
+      BLOCK_ROWS_BEGIN(B0, n)
+        const double pv = P.p[i], qv = P.q[i], yv = P.y[i], rv = P.r[i];
+        const float di = L0.dinv[i];
+        P.y[i] = yv + alpha * pv;
+        const double r = rv - alpha * qv;
+        P.r[i] = r;
+        L0.db[i] = di * static_cast<float>(r);
+        rh += r * r;
+      BLOCK_ROWS_END
+      dummy = 0.0;
+      if (!sync_sum(P, S, flip, rh, dummy)) return;
       pcg_mark(tm, 29, P.timing);
-      cta_total(P.part, 0, tot, sh);
-      rr = tot[0];
+      rr = rh;
       ++total;
       rz_old = rz;
       // stop a little below the target so that the true residual confirms it
@@ -1051,18 +1222,17 @@ __global__ void __launch_bounds__(PCG_BLOCK, PCG_CTAS_PER_SM) k_pcg_amg(PcgParam
   double mx = 0.0;
   if (P.project) {
     double sx = 0.0;
-    PCG_ROWS_BEGIN sx += P.y[row] * P.sdinv[row];
-    PCG_ROWS_END
-    cta_partial(P.part, 1, sx, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    cta_total(P.part, 1, tot, sh);
-    mx = tot[0] / static_cast<double>(n);
+    BLOCK_ROWS_BEGIN(B0, n) sx += P.y[i];
+    BLOCK_ROWS_END
+    dummy = 0.0;
+    if (!sync_sum(P, S, flip, sx, dummy)) return;
+    mx = sx / static_cast<double>(n);
   }
-  PCG_ROWS_BEGIN
-    const double xv = P.y[row] * P.sdinv[row] - mx;
-    P.x[row] = static_cast<TV>(xv);
-    P.y[row] = xv / P.sdinv[row];
-  PCG_ROWS_END
+  BLOCK_ROWS_BEGIN(B0, n)
+    const double xv = P.y[i] - mx;
+    P.x[i] = static_cast<TV>(xv);
+    P.y[i] = xv;
+  BLOCK_ROWS_END
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *P.iters = total;
     *P.resid = bb > 0.0 ? sqrt(rr / bb) : 0.0;
@@ -1088,30 +1258,30 @@ __device__ bool vcycle_r(const PcgParams<TV>& P, int slot, double* sh, unsigned 
   const int NL = P.nlev;
   int ph = 0;
   for (int l = 0; l + 1 < NL; ++l) {
-    const AmgLevelDev& L = P.lv[l];
+    const AmgLevelDev& L = P.L[l];
     pre_a_r<R>(L, rr);
     if (!grid_barrier(cnt, gen, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
     pre_b_r<R>(L, rr);
     if (!grid_barrier(cnt, gen, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
-    restrict_to_r<R>(L, P.lv[l + 1], rr);
+    restrict_to_r<R>(L, P.L[l + 1], rr);
     if (!grid_barrier(cnt, gen, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
   }
-  coarse_solve_r<R>(P.lv[NL - 1], P.cinv, P.nc, P.ldc, rr);
+  coarse_solve_r<R>(P.L[NL - 1], P.cinv, P.nc, P.ldc, rr);
   if (!grid_barrier(cnt, gen, nb, P.err)) return false;
   pcg_mark(tm, ph++, P.timing);
   for (int l = NL - 2; l >= 0; --l) {
-    const AmgLevelDev& L = P.lv[l];
-    prolong_from_r<R>(L, P.lv[l + 1], rr);
+    const AmgLevelDev& L = P.L[l];
+    prolong_from_r<R>(L, P.L[l + 1], rr);
     if (!grid_barrier(cnt, gen, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
     post_c_r<R>(L, rr);
     if (!grid_barrier(cnt, gen, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
     double rz = 0.0, wz = 0.0;
-    post_d_r<R>(L, rr, P.r, P.sdinv, rz, wz, l == 0);
+    post_d_r<R>(L, rr, P.r, P.diag, rz, wz, l == 0);
     if (l == 0) cta_partial(P.part, slot, rz, wz, 0.0, 0.0, sh);
     if (!grid_barrier(cnt, gen, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
@@ -1135,9 +1305,9 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
   unsigned int* cnt = P.bar;
   unsigned int* gen = P.bar + 1;
   const int64_t n = P.n;
-  float* b0 = P.lv[0].b;
-  float* db0 = P.lv[0].db;
-  const float* dinv0 = P.lv[0].dinv;
+  float* b0 = P.L[0].b;
+  float* db0 = P.L[0].db;
+  const float* dinv0 = P.L[0].dinv;
   double tot[4];
   double meanb = 0.0;
   if (P.project && !P.bh_given) {
@@ -1154,16 +1324,15 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
   {
     double bb = 0.0;
     PCG_ROWS_BEGIN
-      const double sd = P.sdinv[row];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int64_t j = r * n + row;
         double bv;
         if (P.bh_given) {
-          bv = P.bh[j] / sd;
+          bv = P.bh[j];
         } else {
           bv = static_cast<double>(P.b[j]) - meanb;
-          P.bh[j] = bv * sd;
+          P.bh[j] = bv;
         }
         if (!P.warm) P.y[j] = 0.0;
         bb += bv * bv;
@@ -1186,7 +1355,7 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
   double rr = 0.0, rr0 = -1.0;
   for (int outer = 0; outer < P.max_outer; ++outer) {
     ++outers;
-    // true residual r = bh - A^ y (FP64) of every block, its unscaled norm, r -> level-0 rhs
+    // true residual r = bh - A y (FP64) of every block, its norm, r -> level-0 rhs
     {
       double rh = 0.0;
       const uint64_t pst = l2_policy_stream(), pkeep = l2_policy_keep();
@@ -1197,29 +1366,28 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
         int k = 0;
         for (; k + 2 <= width; k += 2) {
           const int64_t idx = base + ((int64_t)k << 5) + lane;
-          const double v0 = ld_hint(P.v64 + idx, pst), v1 = ld_hint(P.v64 + idx + 32, pst);
+          const double v0 = ld_hint(P.a64 + idx, pst), v1 = ld_hint(P.a64 + idx + 32, pst);
           const int32_t c0 = ld_hint(P.col + idx, pkeep), c1 = ld_hint(P.col + idx + 32, pkeep);
 #pragma unroll
           for (int r = 0; r < R; ++r) acc[r] += v0 * P.y[r * n + c0] + v1 * P.y[r * n + c1];
         }
         if (k < width) {
           const int64_t idx = base + ((int64_t)k << 5) + lane;
-          const double v = ld_hint(P.v64 + idx, pst);
+          const double v = ld_hint(P.a64 + idx, pst);
           const int32_t c = ld_hint(P.col + idx, pkeep);
 #pragma unroll
           for (int r = 0; r < R; ++r) acc[r] += v * P.y[r * n + c];
         }
         const float di0 = dinv0[row];
-        const double sd = P.sdinv[row], dg = P.diag[row];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const double rv = P.bh[r * n + row] - acc[r];
           const int64_t j = row * R + r;
           P.r[j] = rv;
-          const float rf = static_cast<float>(rv / sd);
+          const float rf = static_cast<float>(rv);
           b0[j] = rf;
           db0[j] = di0 * rf;
-          rh += dg * rv * rv;
+          rh += rv * rv;
         }
       PCG_SLICES_END
       cta_partial(P.part, 0, rh, 0.0, 0.0, 0.0, sh);
@@ -1237,14 +1405,13 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
       const double rz = tot[0];
       const double c = P.project && P.ww > 0.0 ? tot[1] / P.ww : 0.0;
       const double beta = it == 0 ? 0.0 : rz / rz_old;
-      const float* u0 = P.lv[0].x;  // u = D^-1/2 z^ of every block (interleaved)
+      const float* u0 = P.L[0].x;  // u of every block (interleaved)
       double pq = 0.0;
       const uint64_t pkeep = l2_policy_keep();
       PCG_SLICES_BEGIN
         float uf[R];
         load_r<R>(u0, row, uf);
         const double rs = P.rsum[row];
-        const double sd = P.sdinv[row];
         double ui[R], acc[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -1275,10 +1442,8 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const int64_t j = row * R + r;
-          const double av = (acc[r] + rs * ui[r]) * sd;
-          const double z = ui[r] / sd;
-          const double w = 1.0 / sd;
-          const double pv = (z - c * w) + (it == 0 ? 0.0 : beta * P.p[j]);
+          const double av = acc[r] + rs * ui[r];
+          const double pv = (ui[r] - c) + (it == 0 ? 0.0 : beta * P.p[j]);
           const double qv = av + (it == 0 ? 0.0 : beta * P.q[j]);
           P.p[j] = pv;
           P.q[j] = qv;
@@ -1295,7 +1460,6 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
       double rh = 0.0;
       PCG_ROWS_BEGIN
         const float di0 = dinv0[row];
-        const double sd = P.sdinv[row], dg = P.diag[row];
         double pv[R], rv[R], qv[R];
         load_r64<R>(P.p, row, pv);
         load_r64<R>(P.r, row, rv);
@@ -1305,10 +1469,10 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
         for (int r = 0; r < R; ++r) {
           P.y[r * n + row] += alpha * pv[r];
           rv[r] -= alpha * qv[r];
-          const float rf = static_cast<float>(rv[r] / sd);
+          const float rf = static_cast<float>(rv[r]);
           bf[r] = rf;
           dbf[r] = di0 * rf;
-          rh += dg * rv[r] * rv[r];
+          rh += rv[r] * rv[r];
         }
         store_r64<R>(P.r, row, rv);
         store_r<R>(b0, row, bf);
@@ -1328,9 +1492,8 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
   if (P.project) {
     double sx = 0.0;
     PCG_ROWS_BEGIN
-      const double sd = P.sdinv[row];
 #pragma unroll
-      for (int r = 0; r < R; ++r) sx += P.y[r * n + row] * sd;
+      for (int r = 0; r < R; ++r) sx += P.y[r * n + row];
     PCG_ROWS_END
     cta_partial(P.part, 1, sx, 0.0, 0.0, 0.0, sh);
     if (!grid_barrier(cnt, gen, nb, P.err)) return;
@@ -1338,13 +1501,12 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
     mx = tot[0] / static_cast<double>(R * n);
   }
   PCG_ROWS_BEGIN
-    const double sd = P.sdinv[row];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int64_t j = r * n + row;
-      const double xv = P.y[j] * sd - mx;
+      const double xv = P.y[j] - mx;
       P.x[j] = static_cast<TV>(xv);
-      P.y[j] = xv / sd;
+      P.y[j] = xv;
     }
   PCG_ROWS_END
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1410,8 +1572,11 @@ void CgSystem<TM>::enable_amg(const HostSell& hs, const std::vector<int64_t>& ro
       for (int64_t k = L0.P.rp[i]; k < L0.P.rp[i + 1]; ++k) L0.P.v[k] /= std::sqrt(d[i]);
     for (int64_t k = 0; k < static_cast<int64_t>(L0.R.v.size()); ++k) L0.R.v[k] /= std::sqrt(d[L0.R.ci[k]]);
   }
+  int dev;
+  SPX_CUDA(cudaGetDevice(&dev));
+  amg_grid = num_sms(dev) * PCG_CTAS_PER_SM;
   amg = std::make_unique<AmgDevice>();
-  amg->upload(h, s, P.slice_ptr.p, P.col.p, amg_a32.p, P.nslices, reps);
+  amg->upload(h, s, P.slice_ptr.p, P.col.p, amg_a32.p, P.nslices, reps, amg_grid);
   amg_ww = ww;
   amg_singular = singular;
   if (!y64.n) {
@@ -1421,15 +1586,23 @@ void CgSystem<TM>::enable_amg(const HostSell& hs, const std::vector<int64_t>& ro
   if (!bh64.n) bh64.alloc(this->n);
   amg_work.alloc(3 * static_cast<size_t>(this->n));
   amg_work.zero(s);
-  if (!vals64.n) {  // FP64 scaled values (the FP64 CG keeps them in vals)
-    std::vector<double> v(P.len);
-    SPX_CUDA(cudaMemcpy(v.data(), vals.p, P.len * sizeof(double), cudaMemcpyDeviceToHost));
+  {  // unscaled FP64 values (true residual)
+    std::vector<double> v(P.len, 0.0);
+    for (int64_t k = 0; k < static_cast<int64_t>(a.size()); ++k)
+      if (hs.map[k] >= 0) v[hs.map[k]] = a[k];
     vals64.upload(v, s);
+    vals.release();  // the scaled values and vectors belong to the Jacobi solvers
+    work.release();
   }
   SPX_CHECK(reps == 1 || reps == 2 || reps == 4 || reps == 8, "repeated blocks: 1, 2, 4 or 8");
   int per_sm = 0;
-  SPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_amg<double>, PCG_BLOCK, 0));
-  SPX_CHECK(per_sm >= PCG_CTAS_PER_SM, "AMG PCG kernel cannot be resident");
+  if (reps == 1) {
+    plan_resident();
+    for (const void* kk : {reinterpret_cast<const void*>(k_pcg_amg<double>), reinterpret_cast<const void*>(k_pcg_amg<float>)})
+      SPX_CUDA(cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, PCG_DYN_MAX));
+    SPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_amg<double>, PCG_BLOCK, amg->smem_bytes));
+    SPX_CHECK(per_sm >= PCG_CTAS_PER_SM, "AMG PCG kernel cannot be resident");
+  }
   if (reps > 1) {
     const void* kr = reps == 2 ? reinterpret_cast<const void*>(k_pcg_amg_r<double, 2>)
                      : reps == 4 ? reinterpret_cast<const void*>(k_pcg_amg_r<double, 4>)
@@ -1448,9 +1621,6 @@ void CgSystem<TM>::enable_amg(const HostSell& hs, const std::vector<int64_t>& ro
     SPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kr, PCG_BLOCK_R, dyn));
     SPX_CHECK(per_sm >= PCG_CTAS_PER_SM, "AMG PCG kernel (repeated blocks) cannot be resident");
   }
-  int dev;
-  SPX_CUDA(cudaGetDevice(&dev));
-  amg_grid = num_sms(dev) * PCG_CTAS_PER_SM;
   {
     int64_t keep = P.len * static_cast<int64_t>(sizeof(float) + sizeof(int32_t));  // level 0 (shared pattern)
     for (int l = 1; l + 1 < amg->nlev; ++l) keep += amg->A[l].len * static_cast<int64_t>(sizeof(float) + sizeof(int32_t));
@@ -1461,13 +1631,41 @@ void CgSystem<TM>::enable_amg(const HostSell& hs, const std::vector<int64_t>& ro
   SPX_CUDA(cudaStreamSynchronize(s));
 }
 
+// Shared memory of k_pcg_amg, finest level first: the slice bounds of a level (4 bytes a slice),
+// then as many of its entries (FP32 value and column) as still fit.  400x400x2 film: all of
+// level 0 (165 KB a CTA) and part of level 1.
+template <class TM>
+void CgSystem<TM>::plan_resident() {
+  AmgDevice& A = *amg;
+  A.res.assign(A.nlev, AmgResident{-1, 0, 0, 0, 0, 0});
+  int64_t pos = 0;  // words
+  const int64_t lim = PCG_DYN_MAX / 4;
+  for (int l = 0; l + 1 < A.nlev; ++l) {
+    const int64_t words = (A.cnt[l] + 1 + 3) / 4 * 4;
+    const int64_t rwords = ((A.sizes[l + 1] + amg_grid - 1) / amg_grid + 1 + 3) / 4 * 4;
+    if (pos + 2 * words + rwords > lim / 4) break;  // a level of thousands of slices a CTA streams
+    A.res[l].off = static_cast<int32_t>(pos);
+    A.res[l].poff = static_cast<int32_t>(pos + words);
+    A.res[l].roff = static_cast<int32_t>(pos + 2 * words);
+    pos += 2 * words + rwords;
+  }
+  for (int l = 0; l + 1 < A.nlev && A.res[l].off >= 0; ++l) {
+    const int64_t cap = std::min<int64_t>(A.need[l], (lim - pos) / 2 / 32 * 32);
+    A.res[l].val = static_cast<int32_t>(pos);
+    A.res[l].col = static_cast<int32_t>(pos + cap);
+    A.res[l].cap = static_cast<int32_t>(cap);
+    pos += 2 * cap;
+  }
+  A.smem_bytes = static_cast<size_t>(pos) * 4;
+}
+
 template <class TM>
 template <class TV>
 void CgSystem<TM>::launch_amg(const TV* b, TV* x, double rtol, double atol, int maxit, bool warm, bool project,
                               cudaStream_t st, bool bh_given) {
   PcgParams<TV> q;
   q.n = n1; q.nslices = P.nslices; q.sp = P.slice_ptr.p; q.col = P.col.p; q.reps = reps;
-  q.v64 = vals64.p; q.a32 = amg_a32.p; q.rsum = amg_rsum.p; q.sdinv = sdinv64.p; q.diag = diag64.p;
+  q.a64 = vals64.p; q.a32 = amg_a32.p; q.rsum = amg_rsum.p; q.diag = diag64.p;
   q.b = b; q.x = x;
   q.bh = bh64.p; q.y = y64.p;
   q.r = amg_work.p; q.p = amg_work.p + n; q.q = amg_work.p + 2 * n;
@@ -1476,14 +1674,19 @@ void CgSystem<TM>::launch_amg(const TV* b, TV* x, double rtol, double atol, int 
   q.rtol = rtol; q.atol = atol; q.ww = amg_singular ? amg_ww : 0.0;
   q.maxit = maxit; q.max_outer = max_outer; q.warm = warm ? 1 : 0; q.project = project ? 1 : 0;
   q.bh_given = bh_given ? 1 : 0;
-  q.lv = amg->lv.p; q.nlev = amg->nlev; q.cinv = amg->cinv.p; q.nc = amg->nc; q.ldc = amg->ldc;
+  q.nlev = amg->nlev;
+  for (int l = 0; l < amg->nlev; ++l) {
+    q.L[l] = amg->lv[l];
+    q.R[l] = amg->res[l];
+  }
+  q.cinv = amg->cinv.p; q.nc = amg->nc; q.ldc = amg->ldc;
   q.timing = g_pcg_timing.load(std::memory_order_relaxed);
   void* args[] = {&q};
   void* k = reinterpret_cast<void*>(k_pcg_amg<TV>);
   if (reps == 2) k = reinterpret_cast<void*>(k_pcg_amg_r<TV, 2>);
   if (reps == 4) k = reinterpret_cast<void*>(k_pcg_amg_r<TV, 4>);
   if (reps == 8) k = reinterpret_cast<void*>(k_pcg_amg_r<TV, 8>);
-  const size_t dyn = reps > 1 ? static_cast<size_t>(amg->nc) * reps * sizeof(float) : 0;
+  const size_t dyn = reps > 1 ? static_cast<size_t>(amg->nc) * reps * sizeof(float) : amg->smem_bytes;
   SPX_CUDA(cudaLaunchCooperativeKernel(k, dim3(amg_grid), dim3(reps > 1 ? PCG_BLOCK_R : PCG_BLOCK), args, dyn, st));
 }
 

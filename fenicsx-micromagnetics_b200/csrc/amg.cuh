@@ -19,8 +19,6 @@
 // of the level-0 matrix.
 #pragma once
 
-#include <cuda_fp16.h>
-
 #include "spx_internal.cuh"
 
 namespace spx {
@@ -35,7 +33,7 @@ struct CsrHost {
 struct AmgOptions {
   double theta = 0.0;         // strength threshold (0: every nonzero off-diagonal is strong)
   int64_t coarse_max = 2500;  // dense coarsest level (inverted once, applied as a GEMV)
-  int max_levels = 10;
+  int max_levels = 10;        // at most AMG_MAX_LEVELS
   int power_iters = 20;
 };
 
@@ -61,7 +59,6 @@ struct AmgLevelDev {
   const int64_t* sp;       // A: SELL-32
   const int32_t* col;
   const float* val;
-  const __half* val16;     // FP16 copy of val for the cycle's sweeps (null: val)
   const float* dinv;
   int64_t p_nslices;       // P: SELL-32, n rows
   const int64_t* p_sp;
@@ -75,6 +72,15 @@ struct AmgLevelDev {
   float theta, delta, sigma;
 };
 
+constexpr int AMG_MAX_LEVELS = 10;
+
+// Where a CTA of k_pcg_amg keeps its block of a level's matrix (4-byte words from the start of
+// its dynamic shared memory): slice bounds of A at `off` (-1: not kept) and of P at `poff`, row
+// bounds of R at `roff`, values of up to `cap` entries of A at `val`, their columns at `col`.
+struct AmgResident {
+  int32_t off, poff, roff, val, col, cap;
+};
+
 struct AmgDevice {
   int nlev = 0;            // levels 0..nlev-2 are cycled, level nlev-1 is the dense coarsest
   int64_t n0 = 0, nc = 0, ldc = 0;  // ldc: row stride of the coarsest inverse (cinv)
@@ -83,15 +89,19 @@ struct AmgDevice {
   std::vector<DevBuf<int64_t>> rrp;
   std::vector<DevBuf<int32_t>> rcol;
   std::vector<DevBuf<float>> val, pval, rval, dinv, vec;
-  std::vector<DevBuf<__half>> val16;  // FP16 sweep values (SPX_AMG_FP16)
-  DevBuf<AmgLevelDev> lv;
+  std::vector<AmgLevelDev> lv;  // passed to the PCG kernels by value
+  // shared-memory residency of the level matrices (plan_resident): per level the slices and
+  // entries of the largest CTA block, and what of it is kept
+  std::vector<int64_t> cnt, need;
+  std::vector<AmgResident> res;
+  size_t smem_bytes = 0;
   DevBuf<float> cinv;
   std::vector<int64_t> sizes, nnz, pnnz, rnnz;  // per level: rows, nonzeros of A, P, R
   // top0: when set, level 0's matrix is this SELL-32 (slice pointers, columns, FP32 values of
   // nslices0 slices) owned by the caller instead of a copy of lv[0].A
-  // nrep: the cycle runs on nrep identical blocks at once (level vectors of nrep x rows)
+  // grid: CTAs of the PCG kernel; nrep: the cycle runs on nrep identical blocks at once (level vectors of nrep x rows)
   void upload(const AmgHost& h, cudaStream_t s, const int64_t* sp0 = nullptr, const int32_t* col0 = nullptr,
-              const float* val0 = nullptr, int64_t nslices0 = 0, int nrep = 1);
+              const float* val0 = nullptr, int64_t nslices0 = 0, int nrep = 1, int grid = 1);
   int64_t device_bytes() const;
 };
 

@@ -138,7 +138,7 @@ __global__ void k_dense_gemv(int64_t Nb, const double* __restrict__ B, const TV*
 // (the same mean in every CTA, deterministic) and remove the mean from their chunk.
 constexpr int SEG_CH = 8192;
 
-// chunk sums of x (or of y sdinv when y is given: the FP64 state), or of b when x is null
+// chunk sums of x, or of y sdinv when y is given: the FP64 state (of y without sdinv)
 template <class TV>
 __global__ void k_seg_sum(const int64_t* __restrict__ off, int maxch, const TV* __restrict__ x,
                           const double* __restrict__ y, const double* __restrict__ sdinv, double* __restrict__ part) {
@@ -148,7 +148,7 @@ __global__ void k_seg_sum(const int64_t* __restrict__ off, int maxch, const TV* 
   if (a >= end) return;  // uniform per CTA
   const int64_t e = min(end, a + SEG_CH);
   double v = 0.0;
-  for (int64_t i = a + threadIdx.x; i < e; i += blockDim.x) v += y ? y[i] * sdinv[i] : static_cast<double>(x[i]);
+  for (int64_t i = a + threadIdx.x; i < e; i += blockDim.x) v += y ? (sdinv ? y[i] * sdinv[i] : y[i]) : static_cast<double>(x[i]);
   v = block_sum(v, sh);
   if (threadIdx.x == 0) part[static_cast<int64_t>(seg) * maxch + c] = v;
 }
@@ -163,7 +163,7 @@ __device__ __forceinline__ double seg_mean(const int64_t* __restrict__ off, int 
 }
 
 // remove each component's mean from a projected solution (x = y sdinv when the FP64 state y
-// is kept)
+// is kept, x = y when it is kept unscaled: no sdinv)
 template <class TV>
 __global__ void k_seg_center(const int64_t* __restrict__ off, int maxch, const double* __restrict__ part,
                              TV* __restrict__ x, double* __restrict__ y, const double* __restrict__ sdinv) {
@@ -174,16 +174,17 @@ __global__ void k_seg_center(const int64_t* __restrict__ off, int maxch, const d
   const double mean = seg_mean(off, maxch, part, seg);
   for (int64_t i = a + threadIdx.x; i < e; i += blockDim.x) {
     if (y) {
-      const double xv = y[i] * sdinv[i] - mean;
+      const double sd = sdinv ? sdinv[i] : 1.0;
+      const double xv = y[i] * sd - mean;
       x[i] = static_cast<TV>(xv);
-      y[i] = xv / sdinv[i];
+      y[i] = xv / sd;
     } else {
       x[i] = static_cast<TV>(static_cast<double>(x[i]) - mean);
     }
   }
 }
 
-// bh = (b minus its mean over each component) * sdinv, in FP64
+// bh = (b minus its mean over each component) * sdinv (1 without sdinv), in FP64
 template <class TV>
 __global__ void k_seg_center_bh(const int64_t* __restrict__ off, int maxch, const double* __restrict__ part,
                                 const TV* __restrict__ b, const double* __restrict__ sdinv, double* __restrict__ bh) {
@@ -192,7 +193,8 @@ __global__ void k_seg_center_bh(const int64_t* __restrict__ off, int maxch, cons
   if (a >= end) return;
   const int64_t e = min(end, a + SEG_CH);
   const double mean = seg_mean(off, maxch, part, seg);
-  for (int64_t i = a + threadIdx.x; i < e; i += blockDim.x) bh[i] = (static_cast<double>(b[i]) - mean) * sdinv[i];
+  for (int64_t i = a + threadIdx.x; i < e; i += blockDim.x) 
+    bh[i] = (static_cast<double>(b[i]) - mean) * (sdinv ? sdinv[i] : 1.0);
 }
 
 // out = b minus its mean over each component
@@ -629,6 +631,30 @@ int repeated_blocks(const HostFem& fem, const std::vector<int64_t>& off) {
   return static_cast<int>(ns);
 }
 
+// the stiffness CSR without its exact zeros off the diagonal (edges whose dihedral angles are
+// all right ones, about half of the entries of a mesh of cut cubes): the Poisson solvers read
+// their matrices tens of times per solve, and a zero term changes no sum
+struct PoissonCsr {
+  std::vector<int64_t> rp;
+  std::vector<int32_t> ci;
+  std::vector<double> a;
+};
+PoissonCsr drop_zeros(const HostFem& fem) {
+  PoissonCsr o;
+  o.rp.assign(fem.N + 1, 0);
+  o.ci.reserve(fem.col.size());
+  o.a.reserve(fem.col.size());
+  for (int64_t i = 0; i < fem.N; ++i) {
+    for (int64_t k = fem.rowptr[i]; k < fem.rowptr[i + 1]; ++k)
+      if (fem.A[k] != 0.0 || fem.col[k] == i) {
+        o.ci.push_back(fem.col[k]);
+        o.a.push_back(fem.A[k]);
+      }
+    o.rp[i + 1] = static_cast<int64_t>(o.ci.size());
+  }
+  return o;
+}
+
 // ------------------------------------------------------------------ CgSystem
 template <class TM>
 void CgSystem<TM>::setup(const HostSell& s, const std::vector<double>& vals_sell, const std::vector<double>& d,
@@ -745,8 +771,9 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
     k_seg_sum<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, b, nullptr, nullptr, seg_part.p);
     SPX_LAUNCH_CHECK();
   }
+  const double* seg_sd = use_amg ? nullptr : sdinv64.p;  // the AMG PCG keeps its state unscaled
   if (seg && ir) {
-    k_seg_center_bh<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, b, sdinv64.p, bh64.p);
+    k_seg_center_bh<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, b, seg_sd, bh64.p);
     SPX_LAUNCH_CHECK();
   } else if (seg) {
     if (bseg.n < n * sizeof(TV)) bseg.alloc(n * sizeof(TV));
@@ -789,9 +816,9 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
     SPX_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg), dim3(grid), dim3(block), args, 0, st));
   }
   if (project && seg_off.n > 1) {
-    k_seg_sum<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, x, ir ? y64.p : nullptr, sdinv64.p, seg_part.p);
+    k_seg_sum<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, x, ir ? y64.p : nullptr, seg_sd, seg_part.p);
     SPX_LAUNCH_CHECK();
-    k_seg_center<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, x, ir ? y64.p : nullptr, sdinv64.p);
+    k_seg_center<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, x, ir ? y64.p : nullptr, seg_sd);
     SPX_LAUNCH_CHECK();
   }
   if (slot == 0 && stage_correct && have_pred0) {  // stage 1's prediction error
@@ -878,38 +905,27 @@ void DemagCtx<TV, TM>::create(const double* X, int64_t N_, const int32_t* tets, 
     Gv.upload(v, s);
   }
   vol.upload(fem.vol, s);
+  const PoissonCsr K = drop_zeros(fem);
   {
     // an ensemble whose samples all have the same stiffness matrix (a batch of one mesh): the
     // u1 system is that block repeated on the diagonal; its matrix and AMG hierarchy are stored
     // once and the PCG runs on all blocks together (2, 4 or 8 of them)
     const int reps = (opt.backend == 2 && opt.u1_pc == 0) ? repeated_blocks(fem, opt.sample_offsets) : 1;
-    if (reps > 1) {
-      const int64_t n1 = N / reps, nnz1 = fem.rowptr[n1];
-      std::vector<int64_t> rp1(fem.rowptr.begin(), fem.rowptr.begin() + n1 + 1);
-      std::vector<int32_t> col1(fem.col.begin(), fem.col.begin() + nnz1);
-      std::vector<double> A1(fem.A.begin(), fem.A.begin() + nnz1);
-      std::vector<int32_t> rows1(n1);
-      for (int64_t i = 0; i < n1; ++i) rows1[i] = static_cast<int32_t>(i);
-      HostSell hs1;
-      build_sell(rp1, col1, rows1, nullptr, hs1);
-      std::vector<double> a1, d1(n1);
-      sell_values<double>(hs1, A1.data(), 1, true, nnz1, 1.0, a1);
-      for (int64_t i = 0; i < n1; ++i)
-        for (int64_t k = rp1[i]; k < rp1[i + 1]; ++k)
-          if (col1[k] == i) d1[i] = A1[k];
-      cg1.setup(hs1, a1, d1, reps);
-      cg1.enable_amg(hs1, rp1, col1, A1, d1, true, s);
-      SPX_CHECK(static_cast<bool>(cg1.amg), "no AMG hierarchy for the repeated block");
-    } else {
-      std::vector<double> a;
-      sell_values<double>(hsell, fem.A.data(), 1, true, nnz, 1.0, a);
-      std::vector<double> d(N);
-      for (int64_t i = 0; i < N; ++i)
-        for (int64_t k = fem.rowptr[i]; k < fem.rowptr[i + 1]; ++k)
-          if (fem.col[k] == i) d[i] = fem.A[k];
-      cg1.setup(hsell, a, d);
-      if (opt.u1_pc == 0) cg1.enable_amg(hsell, fem.rowptr, fem.col, fem.A, d, true, s);
-    }
+    const int64_t n1 = N / reps, nnz1 = K.rp[n1];
+    const std::vector<int64_t> rp1(K.rp.begin(), K.rp.begin() + n1 + 1);
+    const std::vector<int32_t> col1(K.ci.begin(), K.ci.begin() + nnz1);
+    const std::vector<double> A1(K.a.begin(), K.a.begin() + nnz1);
+    const std::vector<int32_t> rows1(all.begin(), all.begin() + n1);
+    HostSell hs1;
+    build_sell(rp1, col1, rows1, nullptr, hs1);
+    std::vector<double> a1, d1(n1);
+    sell_values<double>(hs1, A1.data(), 1, true, nnz1, 1.0, a1);
+    for (int64_t i = 0; i < n1; ++i)
+      for (int64_t k = rp1[i]; k < rp1[i + 1]; ++k)
+        if (col1[k] == i) d1[i] = A1[k];
+    cg1.setup(hs1, a1, d1, reps);
+    if (opt.u1_pc == 0) cg1.enable_amg(hs1, rp1, col1, A1, d1, true, s);
+    SPX_CHECK(reps == 1 || static_cast<bool>(cg1.amg), "no AMG hierarchy for the repeated block");
     cg1.stage_correct = opt.warm_start == 3;
   }
   std::vector<int32_t> bmap(N, -1), imap(N, -1), inter;
@@ -924,16 +940,17 @@ void DemagCtx<TV, TM>::create(const double* X, int64_t N_, const int32_t* tets, 
   bverts.upload(bd.host.bverts, s);
   if (NI > 0) {
     HostSell sII, sIB;
-    build_sell(fem.rowptr, fem.col, inter, &imap, sII);
-    build_sell(fem.rowptr, fem.col, inter, &bmap, sIB);
+    const int64_t nk = K.rp[N];
+    build_sell(K.rp, K.ci, inter, &imap, sII);
+    build_sell(K.rp, K.ci, inter, &bmap, sIB);
     std::vector<double> aII, aIB;
-    sell_values<double>(sII, fem.A.data(), 1, true, nnz, 1.0, aII);
-    sell_values<double>(sIB, fem.A.data(), 1, true, nnz, 1.0, aIB);
+    sell_values<double>(sII, K.a.data(), 1, true, nk, 1.0, aII);
+    sell_values<double>(sIB, K.a.data(), 1, true, nk, 1.0, aIB);
     std::vector<double> d(NI);
     for (int64_t q = 0; q < NI; ++q) {
       const int64_t i = inter[q];
-      for (int64_t k = fem.rowptr[i]; k < fem.rowptr[i + 1]; ++k)
-        if (fem.col[k] == i) d[q] = fem.A[k];
+      for (int64_t k = K.rp[i]; k < K.rp[i + 1]; ++k)
+        if (K.ci[k] == i) d[q] = K.a[k];
     }
     cg2.setup(sII, aII, d);
     cg2.stage_correct = opt.warm_start == 3;

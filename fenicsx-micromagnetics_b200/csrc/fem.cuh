@@ -103,7 +103,9 @@ struct CgSystem {
   int reps = 1;        // identical diagonal blocks sharing the stored matrix (AMG path only)
   DevSell<TM> P;
   DevBuf<TM> vals;     // scaled values
-  DevBuf<double> vals64, sdinv64, diag64, y64, bh64;  // FP64 data of the refinement solve
+  // FP64 data of the refinement solve: values, solution state and right-hand side are those of
+  // the scaled system for k_cg_ir, unscaled for the AMG PCG
+  DevBuf<double> vals64, sdinv64, diag64, y64, bh64;
   DevBuf<TM> sdinv;    // 1/sqrt(d) (pipelined FP64 path)
   DevBuf<TM> diag;
   DevBuf<char> work;   // solver vectors
@@ -156,6 +158,8 @@ struct CgSystem {
   // build the AMG hierarchy of D^-1/2 A D^-1/2 from the CSR of A (same rows as setup)
   void enable_amg(const HostSell& hs, const std::vector<int64_t>& rowptr, const std::vector<int32_t>& col, const std::vector<double>& a,
                   const std::vector<double>& d, bool singular, cudaStream_t s);
+  // shared-memory plan of k_pcg_amg for this hierarchy
+  void plan_resident();
   template <class TV>
   void launch_amg(const TV* b, TV* x, double rtol, double atol, int maxit, bool warm, bool project, cudaStream_t st,
                   bool bh_given = false);

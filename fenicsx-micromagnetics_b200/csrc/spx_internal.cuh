@@ -250,40 +250,38 @@ __device__ __forceinline__ double block_sum(double v, double* smem) {
 // Grid-wide barrier for cooperative (co-resident) launches.  Every wait is bounded:
 // after `limit` polls the waiting block raises *err and returns false; callers then
 // leave the kernel.  count/gen live in device memory zeroed before the launch.
+__device__ __forceinline__ bool grid_arrive_wait(unsigned int* count, unsigned int nblocks, int* err,
+                                                 long long limit = (1ll << 26)) {
+  // The arrival and the wait of one thread (the CTA's writes must happen before it: bar.sync).
+  // One monotonic arrival counter (zeroed before the launch): the thread adds 1 with release
+  // semantics at GPU scope and polls with acquire loads until the counter reaches the next
+  // multiple of nblocks.  The error word is read every 1024 polls only (a CTA that gave up
+  // never arrives, so the others stop by it or by their own poll limit).
+  unsigned int old;
+  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(count) : "memory");
+  const unsigned int target = (old / nblocks + 1u) * nblocks;
+  for (long long it = 1;; ++it) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+    if (static_cast<int>(v - target) >= 0) return true;
+    if ((it & 1023) == 0 && *reinterpret_cast<volatile int*>(err) != 0) return false;
+    if (it > limit) {
+      atomicCAS(err, 0, ERR_TIMEOUT);
+      return false;
+    }
+    if (it > 4096) __nanosleep(32);
+  }
+}
+
 __device__ __forceinline__ bool grid_barrier(unsigned int* count, unsigned int* gen,
                                              unsigned int nblocks, int* err,
                                              long long limit = (1ll << 26)) {
-  // One monotonic arrival counter (zeroed before the launch): after the CTA's own barrier,
-  // thread 0 adds 1 with release semantics at GPU scope (covering every write the CTA made
-  // before bar.sync) and polls with acquire loads until the counter reaches the next multiple
-  // of nblocks; the closing bar.sync hands the acquired view to the CTA.  The error word is
-  // read every 1024 polls only (a CTA that gave up never arrives, so the others stop by it or
-  // by their own poll limit).  `gen` is not used.
+  // thread 0 arrives and waits between two CTA barriers: the first covers every write the CTA
+  // made, the second hands the acquired view to the CTA.  `gen` is not used.
   (void)gen;
   __shared__ int s_ok;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int old;
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(count) : "memory");
-    const unsigned int target = (old / nblocks + 1u) * nblocks;
-    int ok = 1;
-    for (long long it = 1;; ++it) {
-      unsigned int v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-      if (static_cast<int>(v - target) >= 0) break;
-      if ((it & 1023) == 0 && *reinterpret_cast<volatile int*>(err) != 0) {
-        ok = 0;
-        break;
-      }
-      if (it > limit) {
-        atomicCAS(err, 0, ERR_TIMEOUT);
-        ok = 0;
-        break;
-      }
-      if (it > 4096) __nanosleep(32);
-    }
-    s_ok = ok;
-  }
+  if (threadIdx.x == 0) s_ok = grid_arrive_wait(count, nblocks, err, limit) ? 1 : 0;
   __syncthreads();
   return s_ok != 0;
 }
