@@ -995,6 +995,14 @@ __device__ __forceinline__ bool sync_sum(const PcgParams<TV>& P, PcgShared& S, i
   return S.ok != 0;
 }
 
+// End of one run of PCG iterations: a little below the target, so that the true residual confirms
+// it, or 13 digits below the run's first residual: what is left of the recurrence is then near
+// its rounding error (a warm start 10^3 times worse than zero, with rtol 1e-13, never reached
+// the target within one run), and the next run starts from the true residual.
+__device__ __forceinline__ bool pcg_stop(double rr, double rr_start, double tol2) {
+  return rr <= 0.25 * tol2 || rr <= 1e-26 * rr_start;
+}
+
 // u = V(r): L[0].db holds D^-1 r (FP32) on entry, L[0].x holds u on exit; rz, wz: (r, u), (d, u)
 // over the grid.  nlev >= 2.
 template <class TV>
@@ -1175,6 +1183,7 @@ __global__ void __launch_bounds__(PCG_BLOCK, PCG_CTAS_PER_SM) k_pcg_amg(const __
     }
     if (rr0 < 0.0) rr0 = rr;
     if (rr <= tol2 || total >= P.maxit) break;
+    const double rr_start = rr;
     double rz_old = 1.0;
     for (int it = 0;; ++it) {
       double rz, wz;
@@ -1215,8 +1224,7 @@ __global__ void __launch_bounds__(PCG_BLOCK, PCG_CTAS_PER_SM) k_pcg_amg(const __
       rr = rh;
       ++total;
       rz_old = rz;
-      // stop a little below the target so that the true residual confirms it
-      if (rr <= 0.25 * tol2 || total >= P.maxit) break;
+      if (pcg_stop(rr, rr_start, tol2) || total >= P.maxit) break;
     }
   }
   double mx = 0.0;
@@ -1398,6 +1406,7 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
     rr = tot[0];
     if (rr0 < 0.0) rr0 = rr;
     if (rr <= tol2 || total >= P.maxit) break;
+    const double rr_start = rr;
     double rz_old = 1.0;
     for (int it = 0;; ++it) {
       if (!vcycle_r<TV, R>(P, 2, sh, tm)) return;
@@ -1485,7 +1494,7 @@ __global__ void __launch_bounds__(PCG_BLOCK_R, PCG_CTAS_PER_SM) k_pcg_amg_r(PcgP
       rr = tot[0];
       ++total;
       rz_old = rz;
-      if (rr <= 0.25 * tol2 || total >= P.maxit) break;
+      if (pcg_stop(rr, rr_start, tol2) || total >= P.maxit) break;
     }
   }
   double mx = 0.0;

@@ -2,22 +2,23 @@
 //
 // Pipeline per call (DemagFieldLindholmGPU.compute_vec, gpu/fields/Demag_Lindholm_GPU.py:643-670):
 //   b  = Ms int grad v . m                      k_div   (difference form)
-//   u1 : A u1 = b - mean(b), u1 -= mean(u1)     k_cg / k_cg_ir  (:569-582; PETSc CG+GAMG there)
+//   u1 : A u1 = b - mean(b), u1 -= mean(u1)     k_cg  (:569-582; PETSc CG+GAMG there)
 //   g  = B u1|bnd                               dense GEMV or H-matrix (:585-616)
-//   u2 : A_II u_I = -A_IB g, u2|bnd = g          k_u2rhs + k_cg / k_cg_ir  (:618-640)
+//   u2 : A_II u_I = -A_IB g, u2|bnd = g          k_u2rhs + k_cg  (:618-640)
 //   phi = u1 + u2 ;  H = G phi / V_i            k_grad  (:659-670)
 // The Dirichlet problem is solved on the interior unknowns only; DOLFINx's identity rows for
 // the boundary dofs (assemble_matrix with bcs) give the same interior solution.  CG stops when
 // ||r||_2 <= max(rtol ||b||_2, atol) (unpreconditioned residual, the KSP default test with a
 // zero initial guess) or after maxit.
 //
-// Persistent solvers: one cooperative launch per solve, one CTA of 1024 threads per SM.  Each
-// reduction writes one partial per CTA; after the grid barrier every CTA sums the partials in
-// the same order (deterministic, no contended atomics).  Every barrier wait is bounded.
+// Persistent solvers: one launch per solve (krylov.cuh: one CTA, one cluster or the cooperative
+// grid).  Each reduction sums its partials in the same order everywhere (deterministic, no
+// contended atomics).  Every wait on memory is bounded.
 #include <algorithm>
 #include <cmath>
 
 #include "fem.cuh"
+#include "krylov.cuh"
 
 namespace spx {
 
@@ -197,18 +198,6 @@ __global__ void k_seg_center_bh(const int64_t* __restrict__ off, int maxch, cons
     bh[i] = (static_cast<double>(b[i]) - mean) * (sdinv ? sdinv[i] : 1.0);
 }
 
-// out = b minus its mean over each component
-template <class TV>
-__global__ void k_seg_center_b(const int64_t* __restrict__ off, int maxch, const double* __restrict__ part,
-                               const TV* __restrict__ b, TV* __restrict__ out) {
-  const int seg = blockIdx.y;
-  const int64_t a = off[seg] + static_cast<int64_t>(blockIdx.x) * SEG_CH, end = off[seg + 1];
-  if (a >= end) return;
-  const int64_t e = min(end, a + SEG_CH);
-  const double mean = seg_mean(off, maxch, part, seg);
-  for (int64_t i = a + threadIdx.x; i < e; i += blockDim.x) out[i] = static_cast<TV>(static_cast<double>(b[i]) - mean);
-}
-
 // starting guess: polynomial extrapolation of the stored solutions (order cnt - 1)
 __global__ void k_axpy_sub(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
                            double* __restrict__ out, int mode) {  // mode 0: out = a - b; 1: out += a
@@ -236,198 +225,69 @@ __global__ void k_extrap(int64_t n, ExtrapArgs a, T* __restrict__ out) {
   out[i] = static_cast<T>(v);
 }
 
-constexpr int CG_BLOCK = 1024;
+// ------------------------------------------------------------------ CG with FP64 refinement
+// The scaled system D^-1/2 A D^-1/2 (unit diagonal) by CG in TM (FP32 or FP64) inside FP64
+// iterative refinement, Chronopoulos and Gear's form of CG (both dot products of an iteration in
+// one reduction).
+//
+// What bounds it: a solve takes tens of iterations of 10^3 to 10^5 rows, so the barriers and
+// the load chain between them, not bytes.  The matrix stays in shared memory for the solve.
+//   * A system whose matrix and vectors fit the shared memory of one CTA, or of a cluster of up
+//     to eight, runs there: hardware barriers (40 and 450 cycles against 2,600 over the grid), an
+//     update and a product phase per iteration, the residual gathered from (distributed) shared
+//     memory, the columns kept as its 32-bit addresses.  Bound by shared-memory bandwidth.
+//   * Larger ones run on the grid, one phase per iteration: instead of updating r and q, waiting,
+//     and multiplying, every row forms its neighbours' new residuals itself,
+//       r_j' = r_j - alpha (s_j + beta q_j),   s_i' = sum_j a_ij r_j',
+//     from the records {r, s, q} of the last phase (one 16-byte FP32 gather per entry, two
+//     buffers), which saves one of two grid barriers.  Slices past the shared memory stream
+//     through L2.
+constexpr int CG_BLOCK = 512;
+constexpr int CG_DYN_MAX = 220 * 1024;
+constexpr int CG_SLICES_PER_CTA = 16;  // CTAs of a cluster: one per 16 slices (a round of its warps)
 
-#define CG_ROWS_BEGIN                                               \
-  for (int64_t sl = gw; sl < P.nslices; sl += nw) {                 \
-    const int64_t row = sl * 32 + lane;                             \
-    const int64_t base = P.sp[sl];                                  \
-    const int width = static_cast<int>((P.sp[sl + 1] - base) >> 5); \
-    (void)base; (void)width;                                        \
-    if (row < n) {
-#define CG_ROWS_END \
-  }                 \
+extern __shared__ __align__(16) unsigned char cg_smem[];
+
+template <class TM> struct CgRec;  // r, s, q of one row
+template <> struct CgRec<float> {
+  float r, s, q;
+  using Store = float4;
+  static __device__ __forceinline__ CgRec load(const Store* p) {
+    const float4 v = *p;
+    return {v.x, v.y, v.z};
   }
+  __device__ __forceinline__ void store(Store* p) const { *p = make_float4(r, s, q, 0.0f); }
+};
+struct __align__(32) CgRecD { double r, s, q, pad; };
+template <> struct CgRec<double> {
+  double r, s, q;
+  using Store = CgRecD;
+  static __device__ __forceinline__ CgRec load(const Store* p) {
+    const double2 a = *reinterpret_cast<const double2*>(p);
+    return {a.x, a.y, p->q};
+  }
+  __device__ __forceinline__ void store(Store* p) const {
+    *reinterpret_cast<double2*>(p) = make_double2(r, s);
+    p->q = q;
+  }
+};
 
-// ------------------------------------------------------------------ pipelined FP64 CG
+constexpr int CG_SMEM_VECS = 5;  // r, s, q, p, d of a CTA's rows in shared memory (CTA and cluster teams)
+
+template <class TV, class TM>
 struct CgParams {
   int64_t n, nslices;
   const int64_t* sp;
   const int32_t* col;
-  const double* val;
-  const double* sdinv;
-  const double* diag;
-  const double* b;
-  double* x;
-  double *r, *w0, *w1, *p, *s, *z, *y;
-  double* part;
-  unsigned int* bar;
-  int* err;
-  int* iters;
-  double* resid;
-  unsigned long long* iters_acc;
-  double* res_acc;
-  double rtol, atol;
-  int maxit, warm, project;
-};
-
-__device__ __forceinline__ double spmv64(const CgParams& P, int64_t base, int width, int lane, const double* v) {
-  double acc = 0;
-  for (int k = 0; k < width; ++k) {
-    const int64_t idx = base + ((int64_t)k << 5) + lane;
-    acc += P.val[idx] * v[P.col[idx]];
-  }
-  return acc;
-}
-
-__global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(CgParams P) {
-  __shared__ double sh[160];
-  const unsigned nb = gridDim.x;
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
-  unsigned int* cnt = P.bar;
-  unsigned int* gen = P.bar + 1;
-  const int64_t n = P.n;
-  double tot[4];
-  double meanb = 0.0;
-  if (P.project) {
-    double part = 0.0;
-    CG_ROWS_BEGIN part += P.b[row];
-    CG_ROWS_END
-    cta_partial(P.part, 0, part, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    cta_total(P.part, 0, tot, sh);
-    meanb = tot[0] / static_cast<double>(n);
-  }
-  {
-    double bb = 0.0;
-    CG_ROWS_BEGIN
-      const double bv = P.b[row] - meanb;
-      P.r[row] = bv * P.sdinv[row];
-      P.y[row] = P.warm ? P.x[row] / P.sdinv[row] : 0.0;
-      bb += bv * bv;
-    CG_ROWS_END
-    cta_partial(P.part, 1, bb, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  cta_total(P.part, 1, tot, sh);
-  const double bb = tot[0];
-  // b = 0: the solution is 0 (a warm start would only iterate on rounding noise)
-  const bool warm = P.warm && bb > 0.0;
-  if (P.warm && !warm) {
-    CG_ROWS_BEGIN P.y[row] = 0.0;
-    CG_ROWS_END
-  }
-  if (warm) {
-    CG_ROWS_BEGIN P.r[row] -= spmv64(P, base, width, lane, P.y);
-    CG_ROWS_END
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  {
-    double g = 0.0, dl = 0.0, rh = 0.0;
-    CG_ROWS_BEGIN
-      const double w = spmv64(P, base, width, lane, P.r);
-      P.w0[row] = w;
-      const double rv = P.r[row];
-      g += rv * rv;
-      dl += w * rv;
-      rh += P.diag[row] * rv * rv;
-    CG_ROWS_END
-    cta_partial(P.part, 2, g, dl, rh, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  const double tol2 = fmax(P.rtol * P.rtol * bb, P.atol * P.atol);
-  double gprev = 1.0, aprev = 1.0, rho = 0.0, rho0 = -1.0;
-  int it = 0;
-  for (;; ++it) {
-    cta_total(P.part, 2 + (it & 1), tot, sh);
-    const double gm = tot[0], dl = tot[1];
-    rho = tot[2];
-    if (rho0 < 0.0) rho0 = rho;
-    if (rho <= tol2 || it >= P.maxit || !(gm > 0.0)) break;
-    double beta, alpha;
-    if (it == 0) {
-      beta = 0.0;
-      alpha = gm / dl;
-    } else {
-      beta = gm / gprev;
-      alpha = gm / (dl - beta * gm / aprev);
-    }
-    const double* wc = (it & 1) ? P.w1 : P.w0;
-    double* wn = (it & 1) ? P.w0 : P.w1;
-    double g2 = 0.0, d2 = 0.0, r2 = 0.0;
-    CG_ROWS_BEGIN
-      const double nv = spmv64(P, base, width, lane, wc);
-      const double wv = wc[row];
-      const double rv = P.r[row];
-      double zv, sv, pv;
-      if (it == 0) {
-        zv = nv; sv = wv; pv = rv;
-      } else {
-        zv = nv + beta * P.z[row];
-        sv = wv + beta * P.s[row];
-        pv = rv + beta * P.p[row];
-      }
-      P.z[row] = zv;
-      P.s[row] = sv;
-      P.p[row] = pv;
-      P.y[row] += alpha * pv;
-      const double rn = rv - alpha * sv;
-      const double wnv = wv - alpha * zv;
-      P.r[row] = rn;
-      wn[row] = wnv;
-      g2 += rn * rn;
-      d2 += wnv * rn;
-      r2 += P.diag[row] * rn * rn;
-    CG_ROWS_END
-    // slot 2 + ((it + 1) & 1) was last read at the top of iteration it - 1, a barrier ago
-    cta_partial(P.part, 2 + ((it + 1) & 1), g2, d2, r2, 0.0, sh);
-    gprev = gm;
-    aprev = alpha;
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  double sx = 0.0;
-  CG_ROWS_BEGIN
-    const double xv = P.y[row] * P.sdinv[row];
-    P.x[row] = xv;
-    sx += xv;
-  CG_ROWS_END
-  if (P.project) {
-    cta_partial(P.part, 0, sx, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    cta_total(P.part, 0, tot, sh);
-    const double mx = tot[0] / static_cast<double>(n);
-    CG_ROWS_BEGIN P.x[row] -= mx;
-    CG_ROWS_END
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *P.iters = it;
-    *P.resid = bb > 0.0 ? sqrt(rho / bb) : 0.0;
-    atomicAdd(P.iters_acc, (unsigned long long)it);
-    atomicAdd(P.iters_acc + 1, 1ull);
-    atomicAdd(P.iters_acc + 2, 1ull);
-    if (bb > 0.0) {
-      atomicAdd(P.res_acc, sqrt(fmax(rho0, 0.0) / bb));
-      atomicAdd(P.res_acc + 1, sqrt(rho / bb));
-    }
-  }
-}
-
-// ------------------------------------------------------------------ FP32 CG inside FP64 refinement
-template <class TV>
-struct CgIrParams {
-  int64_t n, nslices;
-  const int64_t* sp;
-  const int32_t* col;
-  const float* v32;
+  const TM* val;
   const double* v64;
   const double* sdinv;
   const double* diag;
   const TV* b;
   TV* x;
   double *bh, *y;
-  float *r, *p, *q, *s, *d;
+  TM *p, *d;
+  typename CgRec<TM>::Store *g0, *g1;
   double* part;
   unsigned int* bar;
   int* err;
@@ -436,166 +296,279 @@ struct CgIrParams {
   unsigned long long* iters_acc;
   double* res_acc;  // [0] sum of initial relative residuals, [1] sum of final ones
   double rtol, atol, inner_rtol;
-  int maxit, max_outer, inner_maxit, warm, project;
-  int bh_given;  // bh already holds the scaled, projected right-hand side (FP64)
+  int maxit, max_outer, warm, project;
+  int bh_given;     // bh already holds the scaled, projected right-hand side (FP64)
+  int32_t off_cap;  // slice bounds kept in shared memory (0: read from sp)
+  int32_t cap;      // entries kept in shared memory per CTA
+  int32_t rows;     // rows of the largest block (CTA and cluster teams)
 };
 
-template <class TV>
-__global__ void __launch_bounds__(CG_BLOCK, 1) k_cg_ir(CgIrParams<TV> P) {
-  __shared__ double sh[160];
-  const unsigned nb = gridDim.x;
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
-  unsigned int* cnt = P.bar;
-  unsigned int* gen = P.bar + 1;
+template <class TV, class TM, int TEAM>
+__global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgParams<TV, TM> P) {
+  using Rec = CgRec<TM>;
+  constexpr bool SM = TEAM != TEAM_GRID;  // records in shared memory
+  constexpr int U = sizeof(TM) == 4 ? 8 : 4;  // records in flight per row (grid)
+  __shared__ TeamShared S;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int64_t n = P.n;
-  double tot[4];
-  double meanb = 0.0;
+  if (TEAM == TEAM_CLUSTER) cluster_sync_all();  // every CTA runs before the first remote store
+  // this CTA's block of slices; bounds, values, columns in shared memory as far as they fit
+  const int64_t s0 = P.nslices * blockIdx.x / gridDim.x;
+  const int cnt = static_cast<int>(P.nslices * (blockIdx.x + 1) / gridDim.x - s0);
+  const int64_t base = P.sp[s0];
+  int32_t* soff = reinterpret_cast<int32_t*>(cg_smem);
+  TM* sval = reinterpret_cast<TM*>(cg_smem + static_cast<size_t>(P.off_cap) * 4);
+  int32_t* scol = reinterpret_cast<int32_t*>(sval + P.cap);
+  const bool off_in = SM || P.off_cap > 0;
+  TM* vr = reinterpret_cast<TM*>(scol + P.cap);
+  TM *vs = vr + P.rows, *vq = vs + P.rows, *vp = vq + P.rows, *vd = vp + P.rows;
+  const unsigned ar = static_cast<unsigned>(__cvta_generic_to_shared(vr));
+  int nres = 0;  // resident slices
+  if (off_in) {
+    for (int k = threadIdx.x; k <= cnt; k += blockDim.x) soff[k] = static_cast<int32_t>(P.sp[s0 + k] - base);
+    __syncthreads();
+    int lo = 0, hi = cnt;  // last bound within the capacity
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (soff[mid] <= P.cap) lo = mid; else hi = mid - 1;
+    }
+    nres = lo;
+    const int m = soff[nres];
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      sval[k] = P.val[base + k];
+      int32_t c = P.col[base + k];
+      if (SM) {  // the address of the column's residual in its owner's shared memory
+        const int64_t own = ((static_cast<int64_t>(c >> 5) + 1) * gridDim.x - 1) / P.nslices;
+        const unsigned a = ar + static_cast<unsigned>(c - 32 * (P.nslices * own / gridDim.x)) * sizeof(TM);
+        c = static_cast<int32_t>(TEAM == TEAM_CLUSTER ? cluster_addr(a, static_cast<unsigned>(own)) : a);
+      }
+      scol[k] = c;
+    }
+  }
+  __syncthreads();
+  auto bounds = [&](int k, int64_t& o, int& width) {
+    if (off_in) {
+      o = soff[k];
+      width = (soff[k + 1] - soff[k]) >> 5;
+    } else {
+      const int64_t a = P.sp[s0 + k];
+      o = a - base;
+      width = static_cast<int>((P.sp[s0 + k + 1] - a) >> 5);
+    }
+  };
+#define CG_ROWS_BEGIN                       \
+  for (int k = wid; k < cnt; k += nw) {     \
+    const int64_t i = (s0 + k) * 32 + lane; \
+    if (i < n) {
+#define CG_ROWS_END \
+  }                 \
+  }
+  int flip = 0;
+  auto sum2 = [&](double& a, double& b) { return team_sum<TEAM>(S, P.part, P.bar, P.err, flip, a, b); };
+  double meanb = 0.0, dummy = 0.0;
   if (P.project && !P.bh_given) {
     double part = 0.0;
-    CG_ROWS_BEGIN part += static_cast<double>(P.b[row]);
+    CG_ROWS_BEGIN part += static_cast<double>(P.b[i]);
     CG_ROWS_END
-    cta_partial(P.part, 0, part, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    cta_total(P.part, 0, tot, sh);
-    meanb = tot[0] / static_cast<double>(n);
+    if (!sum2(part, dummy)) return;
+    meanb = part / static_cast<double>(n);
   }
-  {
-    double bb = 0.0;
-    CG_ROWS_BEGIN
-      double bv;
-      if (P.bh_given) {
-        bv = P.bh[row] / P.sdinv[row];
-      } else {
-        bv = static_cast<double>(P.b[row]) - meanb;
-        P.bh[row] = bv * P.sdinv[row];
-      }
-      if (!P.warm) P.y[row] = 0.0;
-      bb += bv * bv;
-    CG_ROWS_END
-    cta_partial(P.part, 1, bb, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  cta_total(P.part, 1, tot, sh);
-  const double bb = tot[0];
-  if (P.warm && !(bb > 0.0)) {  // b = 0: the solution is 0
-    CG_ROWS_BEGIN P.y[row] = 0.0;
-    CG_ROWS_END
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-  }
-  const double tol2 = fmax(P.rtol * P.rtol * bb, P.atol * P.atol);
+  double bb = 0.0, rho = 0.0, rho0 = -1.0, tol2 = 0.0;
+  bool zero = !P.warm;  // y = 0
   int total = 0, outers = 0;
-  double rho = 0.0, rho0 = -1.0;
   for (int outer = 0; outer < P.max_outer; ++outer) {
     ++outers;
-    // true residual in FP64; inner start r = r64 (FP32), d = 0
+    // true residual in FP64 (and, the first time, the right-hand side); start of the inner solve
     {
-      double rh = 0.0;
+      double rh = 0.0, b2 = 0.0;
       CG_ROWS_BEGIN
-        double acc = 0.0;
-        for (int k = 0; k < width; ++k) {
-          const int64_t idx = base + ((int64_t)k << 5) + lane;
-          acc += P.v64[idx] * P.y[P.col[idx]];
+        const double sd = P.sdinv[i], dg = P.diag[i];
+        double r64;
+        if (outer == 0 && !P.bh_given) {
+          const double bv = static_cast<double>(P.b[i]) - meanb;
+          r64 = bv * sd;
+          P.bh[i] = r64;
+          b2 += bv * bv;
+        } else {
+          r64 = P.bh[i];
+          if (outer == 0) {
+            const double bv = r64 / sd;
+            b2 += bv * bv;
+          }
         }
-        const double r64 = P.bh[row] - acc;
-        rh += P.diag[row] * r64 * r64;
-        P.r[row] = static_cast<float>(r64);
-        P.d[row] = 0.0f;
+        if (zero) {
+          P.y[i] = 0.0;
+        } else {
+          int64_t o;
+          int width;
+          bounds(k, o, width);
+          const double* gv = P.v64 + base + o + lane;
+          const int32_t* gc = P.col + base + o + lane;
+          double acc = 0.0, acc2 = 0.0;
+          for (int j = 0; j < width; j += 4) {
+            double w[4], g[4];
+            int32_t c[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const bool in = j + u < width;
+              c[u] = in ? gc[(j + u) * 32] : 0;
+              w[u] = in ? gv[(j + u) * 32] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) g[u] = j + u < width ? P.y[c[u]] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              acc += w[u] * g[u];
+              acc2 += w[u + 1] * g[u + 1];
+            }
+          }
+          r64 -= acc + acc2;
+        }
+        rh += dg * r64 * r64;
+        if constexpr (SM) {
+          const int row = 32 * k + lane;
+          vr[row] = static_cast<TM>(r64);
+          vs[row] = vq[row] = vp[row] = vd[row] = TM(0);
+        } else {
+          Rec{static_cast<TM>(r64), TM(0), TM(0)}.store(P.g0 + i);
+          P.p[i] = TM(0);
+          P.d[i] = TM(0);
+        }
       CG_ROWS_END
-      cta_partial(P.part, 0, rh, 0.0, 0.0, 0.0, sh);
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
+      if (!sum2(rh, b2)) return;
+      rho = rh;
+      if (outer == 0) {
+        bb = b2;
+        tol2 = fmax(P.rtol * P.rtol * bb, P.atol * P.atol);
+        if (!(bb > 0.0)) {  // b = 0: the solution is 0 (a warm start would only chase rounding noise)
+          CG_ROWS_BEGIN P.y[i] = 0.0;
+          CG_ROWS_END
+          rho = rho0 = 0.0;
+          break;
+        }
+      }
     }
-    cta_total(P.part, 0, tot, sh);
-    rho = tot[0];
+    zero = false;
     if (rho0 < 0.0) rho0 = rho;
     if (rho <= tol2 || total >= P.maxit) break;
     // reduce the residual only as far as the target needs (with a 0.3 margin), at most
-    // by inner_rtol per refinement step (the FP32 inner solve's reliable range)
+    // by inner_rtol per refinement step (the inner solve's reliable range)
     const double need = 0.3 * sqrt(tol2 / rho);
     const double itol = fmax(P.inner_rtol, fmin(need, 0.5));
-    // s = A r, slot 2 <- (r,r), (r,s)
-    {
-      double g = 0.0, dl = 0.0;
-      CG_ROWS_BEGIN
-        float acc = 0.0f;
-        for (int k = 0; k < width; ++k) {
-          const int64_t idx = base + ((int64_t)k << 5) + lane;
-          acc += P.v32[idx] * P.r[P.col[idx]];
+    // alpha = gm / den, den = dl - beta^2 den_prev (= dl - beta gm / alpha_prev): one division
+    // between the sums and the next phase; 1 / gm is formed while they are on their way
+    double g0 = 0.0, ginv = 0.0, den = 0.0;
+    TM a = TM(0), bt = TM(0);
+    for (int it = -1;; ++it) {  // it = -1 (a = bt = 0) only multiplies: s = A r
+      double gm = 0.0, dl = 0.0;
+      if constexpr (SM) {
+        if (it >= 0) {
+          CG_ROWS_BEGIN
+            const int row = 32 * k + lane;
+            const TM qn = vs[row] + bt * vq[row], pn = vr[row] + bt * vp[row];
+            vq[row] = qn;
+            vp[row] = pn;
+            vd[row] += a * pn;
+            vr[row] -= a * qn;
+          CG_ROWS_END
+          if (!team_barrier<TEAM>(P.bar, P.err)) return;
         }
-        P.s[row] = acc;
-        const double rv = P.r[row];
-        g += rv * rv;
-        dl += rv * static_cast<double>(acc);
-      CG_ROWS_END
-      cta_partial(P.part, 2, g, dl, 0.0, 0.0, sh);
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    }
-    double g0 = 0.0, gprev = 1.0, aprev = 1.0;
-    for (int it = 0;; ++it) {
-      cta_total(P.part, 2 + (it & 1), tot, sh);
-      const double gm = tot[0], dl = tot[1];
-      if (it == 0) g0 = gm;
-      if (gm <= itol * itol * g0 || it >= P.inner_maxit || total >= P.maxit || !(gm > 0.0) ||
-          !(dl > 0.0))
-        break;
-      double beta, alpha;
-      if (it == 0) {
-        beta = 0.0;
-        alpha = gm / dl;
+        CG_ROWS_BEGIN
+          const int row = 32 * k + lane, o = soff[k], width = (soff[k + 1] - o) >> 5, so = o + lane;
+          TM acc = TM(0), acc2 = TM(0);
+          for (int j = 0; j < width; j += 8) {
+            unsigned c[8];
+            TM g[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) c[u] = j + u < width ? static_cast<unsigned>(scol[so + (j + u) * 32]) : ar;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (j + u < width) g[u] = team_load<TEAM>(c[u], TM(0));
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (j + u < width) {
+                if (u & 1) acc2 += sval[so + (j + u) * 32] * g[u];
+                else acc += sval[so + (j + u) * 32] * g[u];
+              }
+          }
+          const TM sn = acc + acc2;
+          vs[row] = sn;
+          const double rd = static_cast<double>(vr[row]);
+          gm += rd * rd;
+          dl += rd * static_cast<double>(sn);
+        CG_ROWS_END
       } else {
-        beta = gm / gprev;
-        alpha = gm / (dl - beta * gm / aprev);
+        const typename Rec::Store* cur = (it & 1) ? P.g0 : P.g1;
+        typename Rec::Store* nxt = (it & 1) ? P.g1 : P.g0;
+        CG_ROWS_BEGIN
+          const Rec me = Rec::load(cur + i);
+          const TM pold = P.p[i], dold = P.d[i];
+          int64_t o;
+          int width;
+          bounds(k, o, width);
+          TM acc = TM(0), acc2 = TM(0);
+          const bool res = k < nres;
+          const TM* gv = P.val + base + o + lane;
+          const int32_t* gc = P.col + base + o + lane;
+          const int so = (res ? static_cast<int>(o) : 0) + lane;
+          for (int j = 0; j < width; j += U) {
+            int32_t c[U];
+            Rec g[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              c[u] = j + u < width ? (res ? scol[so + (j + u) * 32] : gc[(j + u) * 32]) : 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (j + u < width) g[u] = Rec::load(cur + c[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (j + u < width) {
+                const TM w = res ? sval[so + (j + u) * 32] : gv[(j + u) * 32];
+                const TM rj = g[u].r - a * (g[u].s + bt * g[u].q);
+                if (u & 1) acc2 += w * rj; else acc += w * rj;
+              }
+          }
+          const TM qn = me.s + bt * me.q, pn = me.r + bt * pold, rn = me.r - a * qn, sn = acc + acc2;
+          Rec{rn, sn, qn}.store(nxt + i);
+          P.p[i] = pn;
+          P.d[i] = dold + a * pn;
+          const double rd = static_cast<double>(rn);
+          gm += rd * rd;
+          dl += rd * static_cast<double>(sn);
+        CG_ROWS_END
       }
-      const float a = static_cast<float>(alpha), bt = static_cast<float>(beta);
-      CG_ROWS_BEGIN
-        const float rv = P.r[row], sv = P.s[row];
-        const float pv = (it == 0) ? rv : rv + bt * P.p[row];
-        const float qv = (it == 0) ? sv : sv + bt * P.q[row];
-        P.p[row] = pv;
-        P.q[row] = qv;
-        P.d[row] += a * pv;
-        P.r[row] = rv - a * qv;
-      CG_ROWS_END
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
-      double g2 = 0.0, d2 = 0.0;
-      CG_ROWS_BEGIN
-        float acc = 0.0f;
-        for (int k = 0; k < width; ++k) {
-          const int64_t idx = base + ((int64_t)k << 5) + lane;
-          acc += P.v32[idx] * P.r[P.col[idx]];
-        }
-        P.s[row] = acc;
-        const double rv = P.r[row];
-        g2 += rv * rv;
-        d2 += rv * static_cast<double>(acc);
-      CG_ROWS_END
-      // slot 2 + ((it+1)&1) was last read at the top of iteration it-1, two barriers ago
-      cta_partial(P.part, 2 + ((it + 1) & 1), g2, d2, 0.0, 0.0, sh);
-      gprev = gm;
-      aprev = alpha;
-      ++total;
-      if (!grid_barrier(cnt, gen, nb, P.err)) return;
+      if (!sum2(gm, dl)) return;
+      if (it < 0) g0 = gm; else ++total;
+      if (gm <= itol * itol * g0 || total >= P.maxit || !(gm > 0.0) || !(dl > 0.0)) break;
+      const double beta = gm * ginv;  // 0 on the first step
+      den = dl - beta * beta * den;
+      bt = static_cast<TM>(beta);
+      a = static_cast<TM>(gm) / static_cast<TM>(den);
+      ginv = 1.0 / gm;
     }
-    CG_ROWS_BEGIN P.y[row] += static_cast<double>(P.d[row]);
+    CG_ROWS_BEGIN
+      if constexpr (SM) P.y[i] += static_cast<double>(vd[32 * k + lane]);
+      else P.y[i] += static_cast<double>(P.d[i]);
     CG_ROWS_END
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
+    if (!team_barrier<TEAM>(P.bar, P.err)) return;
   }
   double mx = 0.0;
   if (P.project) {
     double sx = 0.0;
-    CG_ROWS_BEGIN sx += P.y[row] * P.sdinv[row];
+    CG_ROWS_BEGIN sx += P.y[i] * P.sdinv[i];
     CG_ROWS_END
-    cta_partial(P.part, 1, sx, 0.0, 0.0, 0.0, sh);
-    if (!grid_barrier(cnt, gen, nb, P.err)) return;
-    cta_total(P.part, 1, tot, sh);
-    mx = tot[0] / static_cast<double>(n);
+    dummy = 0.0;
+    if (!sum2(sx, dummy)) return;
+    mx = sx / static_cast<double>(n);
   }
   CG_ROWS_BEGIN
-    const double xv = P.y[row] * P.sdinv[row] - mx;
-    P.x[row] = static_cast<TV>(xv);
-    P.y[row] = xv / P.sdinv[row];
+    const double sd = P.sdinv[i];
+    const double xv = P.y[i] * sd - mx;
+    P.x[i] = static_cast<TV>(xv);
+    if (P.project) P.y[i] = xv / sd;
   CG_ROWS_END
+#undef CG_ROWS_BEGIN
+#undef CG_ROWS_END
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *P.iters = total;
     *P.resid = bb > 0.0 ? sqrt(rho / bb) : 0.0;
@@ -607,6 +580,13 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg_ir(CgIrParams<TV> P) {
       atomicAdd(P.res_acc + 1, sqrt(rho / bb));
     }
   }
+}
+
+template <class TV, class TM>
+const void* cg_kernel(int team) {
+  return team == TEAM_CTA ? reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_CTA>)
+         : team == TEAM_CLUSTER ? reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_CLUSTER>)
+                                : reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_GRID>);
 }
 
 // number of identical diagonal blocks of the FEM system when every sample of an ensemble has
@@ -690,15 +670,11 @@ void CgSystem<TM>::setup(const HostSell& s, const std::vector<double>& vals_sell
     sdinv64.upload(sdr);
     diag64.upload(dr);
   }
-  if (sizeof(TM) == sizeof(float)) {
-    vals64.upload(v64);
-    y64.alloc(n);
-    y64.zero();
-    bh64.alloc(n);
-    work.alloc(5 * static_cast<size_t>(n) * sizeof(float));
-  } else {
-    work.alloc(7 * static_cast<size_t>(n) * sizeof(double));
-  }
+  if (sizeof(TM) == sizeof(float)) vals64.upload(v64);
+  y64.alloc(n);
+  y64.zero();
+  bh64.alloc(n);
+  work.alloc(static_cast<size_t>(n) * (2 * sizeof(TM) + 2 * sizeof(typename CgRec<TM>::Store)));
   bar.alloc(2);
   err.alloc(1);
   iters.alloc(1);
@@ -709,16 +685,48 @@ void CgSystem<TM>::setup(const HostSell& s, const std::vector<double>& vals_sell
   res_acc.zero();
   int dev;
   SPX_CUDA(cudaGetDevice(&dev));
-  int per_sm = 0;
-  block = CG_BLOCK;
-  if (sizeof(TM) == sizeof(float))
-    SPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_ir<double>, CG_BLOCK, 0));
-  else
-    SPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg, CG_BLOCK, 0));
-  SPX_CHECK(per_sm > 0, "CG kernel cannot be resident");
-  const int64_t want = (s.nslices * 32 + CG_BLOCK - 1) / CG_BLOCK;
-  grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(want, num_sms(dev))));
-  part.alloc(4 * 4 * static_cast<size_t>(grid));
+  // the team of k_cg: one CTA or a cluster when matrix and vectors fit their shared memory, else
+  // the grid, a slice a warp.  Per iteration (before: a grid kernel with one or two phases, own
+  // vectors and matrix in global memory): 11 slices on one CTA 1.3 us, 46 slices (20x20x5 box) on
+  // four 1.8 us (10 us on its two CTAs before; 2.3 on eight, 3.0 on two), 132 slices on eight
+  // 2.9 us (grid 4.7), 428 slices on eight 4.5 us (grid 4.5); the grid 4.3-5 us up to 1,200 slices
+  int64_t cnt = 0, need = 0;  // slices and entries of the largest block
+  const int64_t eb = sizeof(TM) + sizeof(int32_t);
+  auto blocks = [&](int g) {
+    grid = g;
+    cnt = need = 0;
+    for (int c = 0; c < g; ++c) {
+      const int64_t a = s.nslices * c / g, e = s.nslices * (c + 1) / g;
+      cnt = std::max(cnt, e - a);
+      need = std::max(need, s.slice_ptr[e] - s.slice_ptr[a]);
+    }
+    off_cap = static_cast<int32_t>((cnt + 1 + 3) / 4 * 4);
+  };
+  auto small_bytes = [&] { return off_cap * 4 + need * eb + cnt * 32 * CG_SMEM_VECS * static_cast<int64_t>(sizeof(TM)); };
+  int g = 1;
+  while (g < TEAM_MAX_CLUSTER && s.nslices > static_cast<int64_t>(g) * CG_SLICES_PER_CTA) g *= 2;
+  blocks(g);
+  while (g < TEAM_MAX_CLUSTER && small_bytes() > CG_DYN_MAX) blocks(g *= 2);
+  if (small_bytes() <= CG_DYN_MAX) {
+    team = g == 1 ? TEAM_CTA : TEAM_CLUSTER;
+    cap = static_cast<int32_t>(need);
+    rows = static_cast<int32_t>(cnt * 32);
+    smem_bytes = static_cast<size_t>(small_bytes());
+    threads = 32 * static_cast<int>(std::min<int64_t>(CG_BLOCK / 32, std::max<int64_t>(cnt, 4)));
+  } else {
+    team = TEAM_GRID;
+    threads = CG_BLOCK;
+    const int64_t per_cta = CG_BLOCK / 32;
+    blocks(static_cast<int>(std::min<int64_t>((s.nslices + per_cta - 1) / per_cta, num_sms(dev))));
+    if (off_cap * 4 > CG_DYN_MAX / 4) off_cap = 0;  // thousands of slices a CTA: all streamed
+    cap = off_cap ? static_cast<int32_t>(std::min<int64_t>(need, (CG_DYN_MAX - off_cap * 4) / eb / 32 * 32)) : 0;
+    rows = 0;
+    smem_bytes = static_cast<size_t>(off_cap) * 4 + static_cast<size_t>(cap) * eb;
+  }
+  part.alloc(4 * 4 * static_cast<size_t>(std::max(grid, num_sms(dev))));
+  std::vector<const void*> ks{cg_kernel<double, TM>(team)};
+  if constexpr (sizeof(TM) == sizeof(float)) ks.push_back(cg_kernel<float, TM>(team));
+  for (const void* k : ks) SPX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_DYN_MAX));
 }
 
 template <class TM>
@@ -730,8 +738,7 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
   last_kind = kind;
   const bool use_amg = static_cast<bool>(amg);
   SPX_CHECK(reps == 1 || use_amg, "a system of repeated blocks is solved by the AMG PCG only");
-  const bool ir = sizeof(TM) == sizeof(float) || use_amg;  // solution state kept in y64
-  SPX_CHECK(ir || sizeof(TV) == sizeof(double), "FP64 CG needs FP64 vectors");
+  SPX_CHECK(sizeof(TM) == sizeof(float) || sizeof(TV) == sizeof(double), "FP64 CG needs FP64 vectors");
   if (slot >= 0) {
     SPX_CHECK(slot < CG_SLOTS, "extrapolation slot out of range");
     for (int k = 0; k < CG_HIST; ++k)
@@ -745,7 +752,7 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
         binom = binom * (ea.cnt - k) / (k + 1);
         ea.w[k] = k < ea.cnt ? ((k % 2) ? -binom : binom) : 0.0;
       }
-      double* target = ir ? y64.p : reinterpret_cast<double*>(x);
+      double* target = y64.p;
       k_extrap<double><<<grid_for(n, 256), 256, 0, st>>>(n, ea, target);
       SPX_LAUNCH_CHECK();
       warm = true;
@@ -772,66 +779,70 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
     SPX_LAUNCH_CHECK();
   }
   const double* seg_sd = use_amg ? nullptr : sdinv64.p;  // the AMG PCG keeps its state unscaled
-  if (seg && ir) {
+  if (seg) {
     k_seg_center_bh<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, b, seg_sd, bh64.p);
     SPX_LAUNCH_CHECK();
-  } else if (seg) {
-    if (bseg.n < n * sizeof(TV)) bseg.alloc(n * sizeof(TV));
-    TV* bc = reinterpret_cast<TV*>(bseg.p);
-    k_seg_center_b<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, b, bc);
-    SPX_LAUNCH_CHECK();
-    b = bc;
   }
   if (use_amg) {
     launch_amg<TV>(b, x, rtol, atol, maxit, warm, project, st, seg);
-  } else if (sizeof(TM) == sizeof(float)) {
-    CgIrParams<TV> q;
+  } else {
+    CgParams<TV, TM> q;
     q.n = n; q.nslices = P.nslices; q.sp = P.slice_ptr.p; q.col = P.col.p;
-    q.v32 = reinterpret_cast<const float*>(vals.p); q.v64 = vals64.p; q.sdinv = sdinv64.p; q.diag = diag64.p;
+    q.val = vals.p; q.sdinv = sdinv64.p; q.diag = diag64.p;
+    q.v64 = sizeof(TM) == sizeof(float) ? vals64.p : reinterpret_cast<const double*>(vals.p);
     q.b = b; q.x = x;
     q.bh = bh64.p; q.y = y64.p;
-    float* Wf = reinterpret_cast<float*>(work.p);
-    q.r = Wf; q.p = Wf + n; q.q = Wf + 2 * n; q.s = Wf + 3 * n; q.d = Wf + 4 * n;
+    using Store = typename CgRec<TM>::Store;
+    q.g0 = reinterpret_cast<Store*>(work.p);
+    q.g1 = q.g0 + n;
+    q.p = reinterpret_cast<TM*>(q.g1 + n);
+    q.d = q.p + n;
     q.part = part.p; q.bar = bar.p; q.err = err.p; q.iters = iters.p; q.resid = resid.p;
     q.iters_acc = iters_acc.p;
     q.res_acc = res_acc.p;
     q.rtol = rtol; q.atol = atol; q.inner_rtol = inner_rtol;
-    q.maxit = maxit; q.max_outer = max_outer; q.inner_maxit = maxit; q.warm = warm ? 1 : 0;
+    q.maxit = maxit; q.max_outer = max_outer; q.warm = warm ? 1 : 0;
     q.bh_given = seg ? 1 : 0;
     q.project = project ? 1 : 0;
-    void* a2[] = {&q};
-    SPX_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg_ir<TV>), dim3(grid), dim3(block), a2, 0, st));
-  } else {
-    CgParams p;
-    p.n = n; p.nslices = P.nslices; p.sp = P.slice_ptr.p; p.col = P.col.p;
-    p.val = reinterpret_cast<const double*>(vals.p); p.sdinv = sdinv64.p; p.diag = diag64.p;
-    p.b = reinterpret_cast<const double*>(b); p.x = reinterpret_cast<double*>(x);
-    double* W = reinterpret_cast<double*>(work.p);
-    p.r = W; p.w0 = W + n; p.w1 = W + 2 * n; p.p = W + 3 * n; p.s = W + 4 * n; p.z = W + 5 * n; p.y = W + 6 * n;
-    p.part = part.p; p.bar = bar.p; p.err = err.p; p.iters = iters.p; p.resid = resid.p;
-    p.iters_acc = iters_acc.p;
-    p.res_acc = res_acc.p;
-    p.rtol = rtol; p.atol = atol; p.maxit = maxit; p.warm = warm ? 1 : 0; p.project = project ? 1 : 0;
-    void* args[] = {&p};
-    SPX_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_cg), dim3(grid), dim3(block), args, 0, st));
+    q.off_cap = off_cap;
+    q.cap = cap;
+    q.rows = rows;
+    const void* k = cg_kernel<TV, TM>(team);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (team == TEAM_CLUSTER) {
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = grid;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    void* args[] = {&q};
+    SPX_CUDA(cudaLaunchKernelExC(&cfg, k, args));
   }
   if (project && seg_off.n > 1) {
-    k_seg_sum<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, x, ir ? y64.p : nullptr, seg_sd, seg_part.p);
+    k_seg_sum<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, x, y64.p, seg_sd, seg_part.p);
     SPX_LAUNCH_CHECK();
-    k_seg_center<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, x, ir ? y64.p : nullptr, seg_sd);
+    k_seg_center<TV><<<sgrid, 256, 0, st>>>(seg_off.p, seg_maxch, seg_part.p, x, y64.p, seg_sd);
     SPX_LAUNCH_CHECK();
   }
   if (slot == 0 && stage_correct && have_pred0) {  // stage 1's prediction error
     if (!delta.n) delta.alloc(n);
-    k_axpy_sub<<<grid_for(n, 256), 256, 0, st>>>(n, ir ? y64.p : reinterpret_cast<const double*>(x), pred0.p,
-                                                 delta.p, 0);
+    k_axpy_sub<<<grid_for(n, 256), 256, 0, st>>>(n, y64.p, pred0.p, delta.p, 0);
     SPX_LAUNCH_CHECK();
     have_delta = true;
     have_pred0 = false;
   }
   if (slot >= 0) {
     double* dst = hist[slot][hhead[slot]].p;
-    const double* src = ir ? y64.p : reinterpret_cast<const double*>(x);
+    const double* src = y64.p;
     SPX_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     hhead[slot] = (hhead[slot] + 1) % CG_HIST;
     hcount[slot] = std::min(CG_HIST, hcount[slot] + 1);

@@ -81,10 +81,9 @@ struct Profiler {
   }
 };
 
-// Scaled SPD system  A^ = D^-1/2 A D^-1/2  on a SELL-32 pattern solved in one cooperative
-// launch: TM = double -> pipelined FP64 CG (one grid barrier per iteration); TM = float ->
-// FP32 single-reduction CG inside FP64 iterative refinement (FP64 values kept for the
-// true residual, FP64 solution state kept between calls).
+// Scaled SPD system  A^ = D^-1/2 A D^-1/2  on a SELL-32 pattern solved in one launch:
+// single-reduction CG in TM inside FP64 iterative refinement (FP64 values for the true
+// residual, FP64 solution state kept between calls).
 //
 // Starting guesses: with `slot` >= 0 the solver keeps the last five solutions returned
 // for that slot (e.g. one slot per RK stage) and starts from their quartic extrapolation
@@ -104,7 +103,7 @@ struct CgSystem {
   DevSell<TM> P;
   DevBuf<TM> vals;     // scaled values
   // FP64 data of the refinement solve: values, solution state and right-hand side are those of
-  // the scaled system for k_cg_ir, unscaled for the AMG PCG
+  // the scaled system for k_cg, unscaled for the AMG PCG
   DevBuf<double> vals64, sdinv64, diag64, y64, bh64;
   DevBuf<TM> sdinv;    // 1/sqrt(d) (pipelined FP64 path)
   DevBuf<TM> diag;
@@ -140,11 +139,13 @@ struct CgSystem {
   int seg_maxch = 0;          // chunks of the largest component (component-mean kernels)
   DevBuf<double> seg_part;    // chunk sums [components][seg_maxch]
   void set_segments(const std::vector<int64_t>& offsets, cudaStream_t s);
-  DevBuf<char> bseg;  // right-hand side with every component's mean removed (TV)
   DevBuf<double> pred0, delta;
-  double inner_rtol = 1e-3;
+  // reduction of one inner solve before its residual is recomputed in FP64
+  double inner_rtol = sizeof(TM) == sizeof(float) ? 1e-3 : 1e-7;
   int max_outer = 10;
-  int grid = 0, block = 0;
+  int grid = 0, threads = 0, team = 0;  // CTAs of k_cg, their threads, which kind of team they form
+  int32_t off_cap = 0, cap = 0, rows = 0;  // slice bounds (words), entries, rows a CTA keeps in shared memory
+  size_t smem_bytes = 0;
   // AMG-preconditioned FP64 CG (k_pcg_amg) instead of the Jacobi solvers when enabled
   std::unique_ptr<AmgDevice> amg;
   DevBuf<double> amg_work;  // r, p, q

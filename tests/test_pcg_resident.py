@@ -1,7 +1,8 @@
-"""The AMG-PCG kernel with its level matrices in shared memory: solutions against the Jacobi solver
-(another kernel, other arithmetic, the same FP64 residual rule) on meshes where a CTA's block of
-slices is empty, partial, wholly resident, or larger than its shared memory; with the stiffness
-matrix's exact zeros (lattice meshes, dropped) and without (moved vertices)."""
+"""The persistent Krylov kernels with their matrices in shared memory, against each other: the
+AMG-PCG and the Jacobi CG (other arithmetic, the same FP64 residual rule) on meshes where a CTA's
+block of slices is empty, partial, wholly resident, or larger than its shared memory, and where
+the Jacobi CG runs on one CTA, on a cluster or on the grid; with the stiffness matrix's exact
+zeros (lattice meshes, dropped) and without (moved vertices)."""
 import numpy as np
 import pytest
 
@@ -19,11 +20,14 @@ def _mesh(nx, ny, nz, jitter):
     return X, T
 
 
-# nodes: 80 (3 slices, most CTAs without rows), 4,736 (one slice a CTA), 4,800 (a partial second
-# one), 29,791 and, 638,976 nodes off the lattice, more matrix than the CTAs' shared memory
-@pytest.mark.parametrize("dims,jitter", [((4, 3, 3), False), ((36, 15, 7), False), ((39, 11, 9), True),
-                                         ((30, 30, 30), True), ((95, 103, 63), True)])
-def test_amg_pcg_matches_jacobi(dims, jitter):
+# nodes: 80 (3 slices: one CTA; most CTAs of the PCG without rows), 1,008 (32 slices: two CTAs),
+# 4,736 (148 slices: one a CTA of the PCG, a cluster of eight), 4,800 (two more slices), 29,791
+# (grid), and 638,976 off the lattice, more matrix than the CTAs' shared memory
+@pytest.mark.parametrize("dims,jitter,precision", [
+    ((4, 3, 3), False, "mixed"), ((4, 3, 3), True, "f64"), ((20, 11, 3), True, "f64"), ((36, 15, 7), False, "mixed"),
+    ((39, 11, 9), True, "f64"), ((30, 30, 30), True, "mixed"), ((30, 30, 30), False, "f64"),
+    ((95, 103, 63), True, "mixed")])
+def test_amg_pcg_matches_jacobi(dims, jitter, precision):
     import torch
     import spinfemx_b200 as spx
     X, T = _mesh(*dims, jitter)
@@ -34,10 +38,10 @@ def test_amg_pcg_matches_jacobi(dims, jitter):
     rtol, u = 1e-10, []
     for pc in ("amg", "jacobi"):
         d = spx.DemagFieldLindholmGPU(X, T, 8e5, boundary_backend="auto", dense_gpu_max_bytes=64 << 20,
-                                      precision="mixed", ksp_rtol_u1=rtol, ksp_rtol_u2=rtol, ksp_atol=0.0,
+                                      precision=precision, ksp_rtol_u1=rtol, ksp_rtol_u2=rtol, ksp_atol=0.0,
                                       ksp_maxit_u1=20000, ksp_maxit_u2=20000, u1_preconditioner=pc)
         d.compute_vec(m, torch.empty_like(m))
-        assert d.last_res_u1 <= rtol
+        assert d.last_res_u1 <= rtol and d.last_res_u2 <= rtol
         u.append(d.potentials()[0])
         del d
     # each solution is off by at most cond(A) rtol, cond(A) below (largest dimension)^2 for the
