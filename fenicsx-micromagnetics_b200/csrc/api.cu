@@ -953,7 +953,8 @@ int spx_hmat_tc_status(spx_hmat hm, int32_t* status) {
   API_BEGIN
   REQUIRE(hm); REQUIRE(status);
   HMatrix& H = hm->h();
-  *status = tc_error(H, 0);
+  const int e = tc_error(H, 0), f = stream_error(H, 0);
+  *status = e ? e : f;
   API_END
 }
 

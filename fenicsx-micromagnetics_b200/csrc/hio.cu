@@ -316,6 +316,7 @@ void hmat_merge(const std::vector<const HMatrix*>& parts, HMatrix& M, cudaStream
   M.zpart_len = zp0;
   M.nunits = u0;
   M.nwarps_z = nwarps;
+  plan_stream(M, units, {}, groups, seg_start, item_ptr, near_begin, near_begin, items, s);
   M.packed = true;
   SPX_CUDA(cudaStreamSynchronize(s));
 }

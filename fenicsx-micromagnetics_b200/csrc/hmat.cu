@@ -15,19 +15,19 @@
 //
 // Kernels (no atomics on data, every output written by exactly one warp or CTA):
 //   k_hgather : x~[i] = src[g(perm[i])]             (fused boundary gather + perm)
-//   k_far_z   : z_b = V_b x~_{J_b} = sum_c x~_c V_b^T[c, :].  Persistent warps over contiguous,
-//               byte-balanced unit ranges; lanes = (16-byte vector of outputs q, phase over
-//               rows c), accumulating in registers across the units of a block; at the
-//               block's last unit in the warp a shuffle sum over the phases writes z_b.  A
-//               block shared by several warps (only at range ends) adds the warps' partials
-//               through an arrival counter: the last arriving warp sums them in contributor
-//               order and resets the counter, so z does not depend on scheduling.
-//   k_rows    : one CTA per row segment; its warps take the segment's items (U tiles with z_b,
-//               near tiles with x~) round-robin, lanes over 16-byte row vectors x phases over
-//               the tile rows, then a fixed-order sum over warps, + diag o x~, scattered to
-//               dst[g(perm[i])].
-// Each warp keeps the factor data of its next units / items moving into L2 with
-// cp.async.bulk.prefetch.L2 (a few units ahead), so its own 16-byte loads mostly hit L2.
+//   k_far_z   : z_b = V_b x~_{J_b} = sum_c x~_c V_b^T[c, :].  Warps over contiguous, byte-balanced
+//               ranges of tiles; lanes = (16-byte vector of outputs q, phase over rows c),
+//               accumulating in registers across the tiles of a block; at the block's last tile
+//               in the warp a shuffle sum over the phases writes z_b.  A block shared by several
+//               warps (only at range ends) adds the warps' partials through an arrival counter:
+//               the last arriving warp sums them in contributor order and resets the counter,
+//               so z does not depend on scheduling.
+//   k_rows    : CTAs over contiguous, byte-balanced ranges of the row segments' tiles (U tiles
+//               with z_b, near tiles with x~), lanes over 16-byte row vectors x phases over the
+//               tile rows, then a fixed-order sum over warps, + diag o x~, scattered to
+//               dst[g(perm[i])]; segments cut by a range end are joined like the blocks.
+// Each warp keeps its next tile moving into L2 with cp.async.bulk.prefetch.L2, and each kernel
+// starts that while the one before it finishes (programmatic dependent launch).
 // Near tiles use compensated (Kahan) accumulation when FP32 accumulates BF16/FP32 data in
 // the mixed-precision form.
 #include <algorithm>
@@ -36,6 +36,7 @@
 
 #include <cuda_fp16.h>
 
+#include "bulk.cuh"
 #include "hmat.cuh"
 
 namespace spx {
@@ -57,10 +58,9 @@ template <> __device__ __forceinline__ double cvt<double, __nv_bfloat16>(__nv_bf
 
 // ------------------------------------------------------------------ packing
 namespace {
-constexpr int Z_WARPS = 8;      // warps per far_z CTA
+constexpr int Z_WARPS = 8;      // warps per CTA and CTAs per SM of the multi-state far_z
 constexpr int Z_CTAS_PER_SM = 4;
 constexpr int SEG_MAX = 64;     // rows per segment
-constexpr int ROWS_WARPS = 8;   // warps per k_rows CTA
 inline int64_t round_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 }  // namespace
 
@@ -93,6 +93,7 @@ __global__ void k_pack(const PackJob* __restrict__ jobs, int64_t njobs, const do
 template <class TS, class TX>
 __global__ void k_hgather(int64_t Nb, const TS* __restrict__ src, const int32_t* __restrict__ gidx,
                           const int32_t* __restrict__ perm, TX* __restrict__ xp) {
+  pdl_trigger();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= Nb) return;
   const int32_t b = perm[i];
@@ -152,11 +153,6 @@ template <>
 __device__ __forceinline__ void v16_elems<float, __nv_bfloat16>(const uint4& v, float out[8]) { bf16x8<float>(v, out); }
 
 
-__device__ __forceinline__ int log2_ceil_le5(int n) {
-  int l = 0;
-  while ((1 << l) < n && l < 5) ++l;
-  return l;
-}
 
 // asynchronous prefetch of a contiguous range into L2 (cp.async.bulk.prefetch.L2; 16-byte
 // aligned address, size a multiple of 16)
@@ -164,90 +160,131 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-#ifndef SPX_Z_PF
-#define SPX_Z_PF 1
-#endif
-#ifndef SPX_R_PF
-#define SPX_R_PF 1
-#endif
-constexpr int Z_PF = SPX_Z_PF;  // units prefetched ahead by each far_z warp
-constexpr int R_PF = SPX_R_PF;  // items prefetched ahead by each rows warp
+// What bounds the apply: HBM reads in flight, not arithmetic (replacing the FMAs by one XOR per
+// entry changes neither kernel's time).  32 warps per SM with four 16-byte loads of a lane in
+// flight and the next tile of each warp on its way into L2: 148 x 32 x 4 KB = 19 MB, three times
+// what 1 us of latency takes at 6.5 TB/s.  Tiles of 16 KB (77 MB of prefetch, over half of L2)
+// cost FP64 factors 18 % and FP32 ones 1-13 %, 2 KB tiles 6-17 %; three CTAs with six loads a lane
+// FP32 8 %.
+// us per product (CTA per row segment, power-of-two lane split, 16 KB units -> this), films of 24,
+// 48, 100, 150, 200, 400 cubes a side: FP32 31.8 -> 24.2, 42.4 -> 29.1, 95 -> 67.6, 167 -> 152,
+// 296 -> 270, 1436 -> 1377..1428; FP64 29.6 -> 23.5, 43.2 -> 29.4, 126 -> 102, 260 -> 230,
+// 465 -> 449, 2359 -> 2295; BF16 28.7 -> 29.6, 44.0 -> 33.5, 86 -> 69, 157 -> 138, 280 -> 249,
+// 1417 -> 1369.
+constexpr int ST_WARPS = 8;          // warps per CTA
+constexpr int ST_CTAS_PER_SM = 4;
+constexpr int ST_TILE = 4096;        // bytes of a tile
+constexpr int ST_THREADS = ST_WARPS * 32;
+constexpr int ST_U = 4;              // 16-byte loads of a lane in flight
 
-template <class TF, class TA, class TX>
-__global__ void __launch_bounds__(Z_WARPS * 32, Z_CTAS_PER_SM)
-    k_far_z(const FarUnit* __restrict__ units, const int32_t* __restrict__ warp_first, int nwarps,
-            const TF* __restrict__ F, const TX* __restrict__ xp, TA* __restrict__ z, TA* __restrict__ zpart,
-            const FarGroup* __restrict__ groups, unsigned int* __restrict__ gcnt) {
-  constexpr int E = V16<TF>::E;
-  using VT = typename V16<TF>::T;
-  using TP = TA;
-  const int wg = static_cast<int>((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5);
-  if (wg >= nwarps) return;  // uniform per warp
+// acc[t] += sum over rows q < len of tile[q][vl E + t] v[q].  Lanes: the nv 16-byte vectors of a row
+// times P = 32 / nv phases over the rows (lane = ph nv + vl; lanes past P nv idle), ST_U rows of a
+// phase in flight.  A split into powers of two (nv rounded up) would leave a quarter of the lanes
+// idle at rank 24, three eighths at 40 rows.
+template <class T, class TA, class TV, int E, bool KAHAN>
+__device__ __forceinline__ void tile_dot(const T* tile_t, const TV* v, int len, int nv, int P, int vl, int ph,
+                                         TA (&acc)[E], TA (&cmp)[E]) {
+  using VT = typename V16<T>::T;
+  const VT* tile = reinterpret_cast<const VT*>(tile_t) + ph * nv + vl;
+  const int st = P * nv;
+  v += ph;
+  auto add = [&](const VT& w, TA a) {
+    TA e[E];
+    v16_elems<TA, T>(w, e);
+#pragma unroll
+    for (int t = 0; t < E; ++t) {
+      if (KAHAN) {
+        const TA y = e[t] * a - cmp[t];
+        const TA s = acc[t] + y;
+        cmp[t] = (s - acc[t]) - y;
+        acc[t] = s;
+      } else {
+        acc[t] += e[t] * a;
+      }
+    }
+  };
+  int q = ph;
+  for (; q + (ST_U - 1) * P < len; q += ST_U * P) {
+    VT w[ST_U];
+    TA a[ST_U];
+#pragma unroll
+    for (int u = 0; u < ST_U; ++u) {
+      w[u] = tile[u * st];
+      a[u] = static_cast<TA>(v[u * P]);
+    }
+#pragma unroll
+    for (int u = 0; u < ST_U; ++u) add(w[u], a[u]);
+    tile += ST_U * st;
+    v += ST_U * P;
+  }
+  for (; q < len; q += P) {
+    add(*tile, static_cast<TA>(*v));
+    tile += st;
+    v += P;
+  }
+}
+// the sum over the phases, in lanes of phase 0: one after the other for a few phases, else a tree
+// (halves of the next power of two first)
+template <class TA>
+__device__ __forceinline__ TA phase_sum(TA a, int nv, int P, int ph) {
   const int lane = threadIdx.x & 31;
-  const int u1 = warp_first[wg + 1];
+  TA y = a;
+  if (P <= 6) {  // uniform
+    for (int p = 1; p < P; ++p) y += __shfl_sync(0xffffffffu, a, lane + p * nv);
+    return y;
+  }
+  for (int s = 16; s > 0; s >>= 1)
+    if (s < P) {
+      const TA t = __shfl_sync(0xffffffffu, y, lane + s * nv);
+      if (ph < s && ph + s < P) y += t;
+    }
+  return y;
+}
+
+// z_b = V_b x~: tiles of a block's V^T dealt to warps in contiguous ranges of about equal bytes.
+template <class TF, class TA>
+__global__ void __launch_bounds__(ST_THREADS, ST_CTAS_PER_SM)
+    k_far_z(const StUnit* __restrict__ units, const int32_t* __restrict__ warp_first, int nwarps,
+            const TF* __restrict__ F, const TA* __restrict__ xp, TA* __restrict__ z, TA* __restrict__ zpart,
+            const FarGroup* __restrict__ groups, unsigned int* __restrict__ gcnt, const double* __restrict__ zscale) {
+  constexpr int E = V16<TF>::E;
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, wg = blockIdx.x * ST_WARPS + (threadIdx.x >> 5);
+  if (wg >= nwarps) return;
   int u = warp_first[wg];
-  FarUnit nxt;
-  if (u < u1) {
+  const int u1 = warp_first[wg + 1];
+  StUnit nxt;
+  if (u < u1) {  // the factors do not depend on the kernel before; x~ does
     nxt = units[u];
     if (lane == 0) prefetch_l2(F + nxt.voff, static_cast<uint32_t>(nxt.nc) * nxt.ldk * sizeof(TF));
   }
-  TA acc[E];
+  pdl_wait();
+  TA acc[E], cmp[E];
 #pragma unroll
   for (int t = 0; t < E; ++t) acc[t] = TA(0);
   for (; u < u1; ++u) {
-    const FarUnit U = nxt;
-    if (u + 1 < u1) nxt = units[u + 1];  // descriptor of the next unit in flight
-    const int nvq = U.ldk / E;
-    const int lg = log2_ceil_le5(nvq);
-    const int G = 1 << lg, P = 32 >> lg;
-    const int vl = lane & (G - 1), ph = lane >> lg;
-    if (vl < nvq) {
-      const VT* tile = reinterpret_cast<const VT*>(F + U.voff) + vl;
-      const TX* x = xp + U.xc;
-      int c = ph;
-      for (; c + 3 * P < U.nc; c += 4 * P) {
-        VT w[4];
-        TP a[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          w[i] = tile[static_cast<int64_t>(c + i * P) * nvq];
-          a[i] = static_cast<TP>(x[c + i * P]);
-        }
-        TP ps[E];
-#pragma unroll
-        for (int t = 0; t < E; ++t) ps[t] = TP(0);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          TP e[E];
-          v16_elems<TP, TF>(w[i], e);
-#pragma unroll
-          for (int t = 0; t < E; ++t) ps[t] += e[t] * a[i];
-        }
-#pragma unroll
-        for (int t = 0; t < E; ++t) acc[t] += static_cast<TA>(ps[t]);
-      }
-      for (; c < U.nc; c += P) {
-        TP e[E];
-        v16_elems<TP, TF>(tile[static_cast<int64_t>(c) * nvq], e);
-        const TP a = static_cast<TP>(x[c]);
-#pragma unroll
-        for (int t = 0; t < E; ++t) acc[t] += static_cast<TA>(e[t] * a);
-      }
-    }
-    if (lane == 0 && u + 1 < u1)  // the next unit's V^T rows into L2
+    const StUnit U = nxt;
+    if (u + 1 < u1) nxt = units[u + 1];  // descriptor of the next tile in flight
+    const int nvq = U.ldk / E, P = U.phases;  // nvq <= 32
+    const int ph = (lane * U.magic) >> 16, vl = lane - ph * nvq;  // lane / nvq
+    if (ph < P) tile_dot<TF, TA, TA, E, false>(F + U.voff, xp + U.xc, U.nc, nvq, P, vl, ph, acc, cmp);
+    if (lane == 0 && u + 1 < u1)  // the next tile into L2
       prefetch_l2(F + nxt.voff, static_cast<uint32_t>(nxt.nc) * nxt.ldk * sizeof(TF));
-    const int fl = U.flags & 3;
+    const int fl = U.flags;
     if (fl == 0) continue;
     // the block ends in this warp: sum over the phases, write its k rows
 #pragma unroll
-    for (int t = 0; t < E; ++t)
-      for (int o = G; o < 32; o <<= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+    for (int t = 0; t < E; ++t) acc[t] = phase_sum(acc[t], nvq, P, ph);
     TA* out = fl == 1 ? z : zpart;
-    if (ph == 0 && vl < nvq) {
+    if (ph == 0) {
 #pragma unroll
       for (int t = 0; t < E; ++t) {
         const int q = vl * E + t;
-        if (q < U.k) out[U.zout + q] = acc[t];
+        if (q < U.k) {
+          TA v = acc[t];
+          if (zscale && fl == 1) v *= static_cast<TA>(zscale[U.zout + q]);
+          out[U.zout + q] = v;
+        }
       }
     }
 #pragma unroll
@@ -264,6 +301,7 @@ __global__ void __launch_bounds__(Z_WARPS * 32, Z_CTAS_PER_SM)
         for (int q = lane; q < Gp.k; q += 32) {
           TA sum = TA(0);
           for (int cc = 0; cc < Gp.ncontrib; ++cc) sum += __ldcg(zpart + Gp.pbase + cc * U.ldk + q);
+          if (zscale) sum *= static_cast<TA>(zscale[Gp.zdst + q]);
           z[Gp.zdst + q] = sum;
         }
         if (lane == 0) atomicExch(gcnt + U.grp, 0u);
@@ -272,149 +310,137 @@ __global__ void __launch_bounds__(Z_WARPS * 32, Z_CTAS_PER_SM)
   }
 }
 
-// Accumulate one warp's share of a segment's items: item it covers tile rows q < len of
-// ld = round_up(nr, E) entries; row q is multiplied by vs[item.src + q].
-template <class T, class TA, class TV>
-__device__ __forceinline__ void rows_items(const RowItem* __restrict__ items, int64_t first, int64_t end,
-                                           const T* __restrict__ base, const TV* __restrict__ vs, int nr,
-                                           TA* __restrict__ part, int lane, bool kahan,
-                                           const double* __restrict__ vscale = nullptr) {
-  constexpr int E = V16<T>::E;
-  using VT = typename V16<T>::T;
-  const int nvec = (nr + E - 1) / E;
-  const int lg = log2_ceil_le5(nvec);
-  const int G = 1 << lg, P = 32 >> lg;
-  const int vl = lane & (G - 1), ph = lane >> lg;
-  TA acc[E], cmp[E];
-#pragma unroll
-  for (int t = 0; t < E; ++t) acc[t] = cmp[t] = TA(0);
-  using TP = TA;
-  const bool active = vl < nvec;
-  RowItem nxt;
-  if (first < end) nxt = items[first];
-  if (lane < R_PF) {  // the first items' tiles into L2
-    const int64_t f = first + static_cast<int64_t>(lane) * ROWS_WARPS;
-    if (f < end) {
-      const RowItem P = items[f];
-      prefetch_l2(base + P.off, static_cast<uint32_t>(P.len) * static_cast<uint32_t>(nvec) * 16u);
-    }
-  }
-  for (int64_t it = first; it < end; it += ROWS_WARPS) {
-    const RowItem I = nxt;
-    if (it + ROWS_WARPS < end) nxt = items[it + ROWS_WARPS];
-    const int64_t fp = it + static_cast<int64_t>(R_PF) * ROWS_WARPS;
-    if (lane == 0 && fp < end) {
-      const RowItem P = items[fp];
-      prefetch_l2(base + P.off, static_cast<uint32_t>(P.len) * static_cast<uint32_t>(nvec) * 16u);
-    }
-    if (!active) continue;
-    const VT* tile = reinterpret_cast<const VT*>(base + I.off) + vl;
-    const TV* v = vs + I.src;
-    const double* sc = vscale ? vscale + I.src : nullptr;
-    int q = ph;
-    for (; q + 3 * P < I.len; q += 4 * P) {
-      VT w[4];
-      TA a[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        w[u] = tile[static_cast<int64_t>(q + u * P) * nvec];
-        a[u] = static_cast<TA>(v[q + u * P]);
-        if (sc) a[u] *= static_cast<TA>(sc[q + u * P]);
-      }
-      if (kahan) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          TA e[E];
-          v16_elems<TA, T>(w[u], e);
-#pragma unroll
-          for (int t = 0; t < E; ++t) {
-            const TA y = e[t] * a[u] - cmp[t];
-            const TA s = acc[t] + y;
-            cmp[t] = (s - acc[t]) - y;
-            acc[t] = s;
-          }
-        }
-      } else {
-        TP ps[E];
-#pragma unroll
-        for (int t = 0; t < E; ++t) ps[t] = TP(0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          TP e[E];
-          v16_elems<TP, T>(w[u], e);
-          const TP au = static_cast<TP>(a[u]);
-#pragma unroll
-          for (int t = 0; t < E; ++t) ps[t] += e[t] * au;
-        }
-#pragma unroll
-        for (int t = 0; t < E; ++t) acc[t] += static_cast<TA>(ps[t]);
-      }
-    }
-    for (; q < I.len; q += P) {
-      const VT w = tile[static_cast<int64_t>(q) * nvec];
-      const TA a = static_cast<TA>(v[q]) * (sc ? static_cast<TA>(sc[q]) : TA(1));
-      TA e[E];
-      v16_elems<TA, T>(w, e);
-      if (kahan) {
-#pragma unroll
-        for (int t = 0; t < E; ++t) {
-          const TA y = e[t] * a - cmp[t];
-          const TA s = acc[t] + y;
-          cmp[t] = (s - acc[t]) - y;
-          acc[t] = s;
-        }
-      } else {
-#pragma unroll
-        for (int t = 0; t < E; ++t) acc[t] += e[t] * a;
-      }
-    }
-  }
+// sum over the phases into the warp's rows of the portion (set: first drain of the portion), and
+// clear the accumulators
+template <class TA, int E>
+__device__ __forceinline__ void tile_drain(TA (&acc)[E], TA (&cmp)[E], int nr, int nv, int P, int vl, int ph, TA* part,
+                                           bool set) {
 #pragma unroll
   for (int t = 0; t < E; ++t) {
-    TA y = acc[t] - cmp[t];
-    for (int o = G; o < 32; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-    acc[t] = y;
-  }
-  if (ph == 0 && active) {
-#pragma unroll
-    for (int t = 0; t < E; ++t) {
-      const int r = vl * E + t;
-      if (r < nr) part[r] += acc[t];
+    const TA y = phase_sum(acc[t] - cmp[t], nv, P, ph);
+    if (ph == 0 && vl * E + t < nr) {
+      TA* p = part + vl * E + t;
+      *p = set ? y : *p + y;
     }
+    acc[t] = cmp[t] = TA(0);
   }
   __syncwarp();
 }
 
-template <class TF, class TN, class TA, class TX, class TD>
-__global__ void __launch_bounds__(ROWS_WARPS * 32) k_rows(
-    const int32_t* __restrict__ seg_start, const int64_t* __restrict__ item_ptr,
-    const int64_t* __restrict__ near_begin, const RowItem* __restrict__ items, const TF* __restrict__ F,
-    const TN* __restrict__ Nt, const TA* __restrict__ z, const TX* __restrict__ xp,
-    const double* __restrict__ diag, const int32_t* __restrict__ perm, const int32_t* __restrict__ gidx,
-    TD* __restrict__ dst, const TD* __restrict__ add, TD* __restrict__ yb, int kahan,
-    const int64_t* __restrict__ half_begin, const __half* __restrict__ Fh, const double* __restrict__ zscale) {
-  __shared__ TA part[ROWS_WARPS][SEG_MAX];
-  const int sgm = blockIdx.x;
-  const int r0 = seg_start[sgm], nr = seg_start[sgm + 1] - r0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = lane; r < SEG_MAX; r += 32) part[warp][r] = TA(0);
-  __syncwarp();
-  const int64_t i0 = item_ptr[sgm], im = near_begin[sgm], i1 = item_ptr[sgm + 1];
-  const int64_t ih = half_begin ? half_begin[sgm] : im;
-  rows_items<TF, TA, TA>(items, i0 + warp, ih, F, z, nr, part[warp], lane, false);
-  if (ih < im) rows_items<__half, TA, TA>(items, ih + warp, im, Fh, z, nr, part[warp], lane, false, zscale);
-  rows_items<TN, TA, TX>(items, im + warp, i1, Nt, xp, nr, part[warp], lane, kahan != 0);
+// the chunks c, c + ST_WARPS, ... < end of one type: tile rows times v, into acc
+template <class T, class TA, int E, bool KAHAN>
+__device__ __forceinline__ void chunks_dot(const StChunk* __restrict__ chunks, int& c, int end, StChunk& nxt, int last,
+                                           const T* __restrict__ base, const TA* __restrict__ v, int type, int nv, int P,
+                                           int vl, int ph, int lane, TA (&acc)[E], TA (&cmp)[E]) {
+  for (; c < end && nxt.type == type; c += ST_WARPS) {
+    const StChunk C = nxt;
+    if (c + ST_WARPS < last) nxt = chunks[c + ST_WARPS];
+    if (lane == 0 && c + ST_WARPS < last && nxt.type == type)  // the next tile into L2
+      prefetch_l2(base + nxt.off, static_cast<uint32_t>(nxt.len) * nxt.ld * sizeof(T));
+    if (ph < P) tile_dot<T, TA, TA, E, KAHAN>(base + C.off, v + C.src, C.len, nv, P, vl, ph, acc, cmp);
+  }
+}
+
+// y = diag x~ + U z + Near x~.  Every CTA takes a contiguous range of chunks (tiles, in segment
+// order), balanced by bytes over the CTAs whatever the segments' sizes; its warps take the
+// range's chunks round-robin.  A portion is the part of a segment inside the range: at its end
+// each warp leaves its sums in shared memory and goes on, and one warp (they take turns) adds
+// them in warp order and writes the rows, or, for a segment shared by several CTAs, leaves a
+// partial that the last of them adds up in portion order.
+template <class TF, class TN, class TA, class TD>
+__global__ void __launch_bounds__(ST_THREADS, ST_CTAS_PER_SM) k_rows(
+    const StPortion* __restrict__ portions, const int32_t* __restrict__ cta_first, const StChunk* __restrict__ chunks,
+    const TF* __restrict__ F, const TN* __restrict__ Nt, const __half* __restrict__ Fh, const TA* __restrict__ z,
+    const TA* __restrict__ xp, const double* __restrict__ diag, const int32_t* __restrict__ perm,
+    const int32_t* __restrict__ gidx, TD* __restrict__ dst, const TD* __restrict__ add, TD* __restrict__ yb,
+    const int2* __restrict__ groups, unsigned int* __restrict__ gcnt, TA* __restrict__ ypart, int* __restrict__ err) {
+  constexpr int EF = V16<TF>::E, EN = V16<TN>::E, EH = V16<__half>::E;
+  constexpr bool KAHAN = sizeof(TA) == sizeof(float) && sizeof(TF) < sizeof(double);
+  __shared__ TA part[2][ST_WARPS][SEG_MAX];
+  __shared__ __align__(8) uint64_t pfull[2], pfree[2];  // partial sums of a portion complete / read
+  if (threadIdx.x < 2) {
+    mbar_init(&pfull[threadIdx.x], ST_WARPS);
+    mbar_init(&pfree[threadIdx.x], 1);
+    fence_mbar_init();
+  }
   __syncthreads();
-  for (int r = threadIdx.x; r < nr; r += blockDim.x) {
-    const int64_t i = r0 + r;
-    TA y = static_cast<TA>(diag[i]) * static_cast<TA>(xp[i]);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p0 = cta_first[blockIdx.x], p1 = cta_first[blockIdx.x + 1];
+  if (p0 >= p1) return;  // uniform per CTA
+  const int c1 = portions[p1 - 1].c1;
+  int c = portions[p0].c0 + warp;
+  StChunk nxt;
+  if (c < c1) {
+    nxt = chunks[c];
+    if (lane == 0) {
+      const uint32_t n = static_cast<uint32_t>(nxt.len) * nxt.ld;
+      if (nxt.type == 0) prefetch_l2(F + nxt.off, n * static_cast<uint32_t>(sizeof(TF)));
+      else if (nxt.type == 2) prefetch_l2(Nt + nxt.off, n * static_cast<uint32_t>(sizeof(TN)));
+    }
+  }
+  pdl_wait();  // z and x~ are complete
+  for (int p = p0; p < p1; ++p) {
+    const StPortion Q = portions[p];
+    const int nr = Q.nr;
+    const int k = p - p0, b = k & 1;
+    const uint32_t use = static_cast<uint32_t>(k >> 1) & 1u;  // parity of this use of buffer b
+    TA* mine = part[b][warp];
+    bool set = true;
+    auto turn = [&](auto typ, auto kah, int type, const auto* base, const TA* v) {
+      using T = decltype(typ);
+      constexpr int E = V16<T>::E;
+      const int nv = (nr + E - 1) / E, P = 32 / nv, ph = lane / nv, vl = lane - ph * nv;
+      TA acc[E], cmp[E];
 #pragma unroll
-    for (int w = 0; w < ROWS_WARPS; ++w) y += part[w][r];
-    const int32_t b = perm[i];
-    const int64_t o = gidx ? gidx[b] : b;
-    const TD yv = static_cast<TD>(y);
-    dst[o] = add ? static_cast<TD>(add[o] + yv) : yv;
-    if (yb) yb[b] = yv;
+      for (int t = 0; t < E; ++t) acc[t] = cmp[t] = TA(0);
+      chunks_dot<T, TA, E, decltype(kah)::value>(chunks, c, Q.c1, nxt, c1, base, v, type, nv, P, vl, ph, lane, acc, cmp);
+      if (set && k >= 2 && !mbar_wait(&pfree[b], use ^ 1u) && lane == 0) atomicCAS(err, 0, ERR_TIMEOUT);
+      tile_drain<TA, E>(acc, cmp, nr, nv, P, vl, ph, mine, set);
+      set = false;
+    };
+    turn(TF{}, std::false_type{}, 0, F, z);
+    if (Fh && c < Q.c1 && nxt.type == 1) turn(__half{}, std::false_type{}, 1, Fh, z);
+    if (c < Q.c1 && nxt.type == 2) turn(TN{}, std::integral_constant<bool, KAHAN>{}, 2, Nt, xp);
+    if (lane == 0) mbar_arrive(&pfull[b]);
+    if (k % ST_WARPS != warp) continue;
+    if (!mbar_wait(&pfull[b], use) && lane == 0) atomicCAS(err, 0, ERR_TIMEOUT);
+    TA y[2] = {TA(0), TA(0)};  // rows lane, lane + 32
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (lane + 32 * h < nr)
+        for (int w = 0; w < ST_WARPS; ++w) y[h] += part[b][w][lane + 32 * h];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&pfree[b]);
+    if (Q.grp >= 0) {  // segment shared with other CTAs: the last portion adds the partials up
+      const int2 G = groups[Q.grp];  // first partial, number of them
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (lane + 32 * h < nr) ypart[static_cast<int64_t>(Q.slot) * SEG_MAX + lane + 32 * h] = y[h];
+      __threadfence();
+      __syncwarp();
+      int last = 0;
+      if (lane == 0) last = atomicAdd(gcnt + Q.grp, 1u) == static_cast<unsigned>(G.y) - 1u ? 1 : 0;
+      if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+      __threadfence();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        y[h] = TA(0);
+        if (lane + 32 * h < nr)
+          for (int g = 0; g < G.y; ++g) y[h] += __ldcg(ypart + static_cast<int64_t>(G.x + g) * SEG_MAX + lane + 32 * h);
+      }
+      if (lane == 0) atomicExch(gcnt + Q.grp, 0u);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = lane + 32 * h;
+      if (r >= nr) continue;
+      const int64_t i = Q.r0 + r;
+      const int32_t bi = perm[i];
+      const int64_t o = gidx ? gidx[bi] : bi;
+      const TD yv = static_cast<TD>(y[h] + static_cast<TA>(diag[i]) * xp[i]);
+      dst[o] = add ? static_cast<TD>(add[o] + yv) : yv;
+      if (yb) yb[bi] = yv;
+    }
   }
 }
 
@@ -489,6 +515,225 @@ std::vector<int32_t> plan_units(std::vector<FarUnit>& units, size_t elem_bytes, 
   return wf;
 }
 
+// The stream plan of the single-vector apply, from the packing's units and segments: V^T units
+// cut to tiles of at most ST_TILE bytes and dealt to the warps of ST_CTAS_PER_SM CTAs per SM; row
+// items cut the same way into chunks, in segment order, dealt to as many CTAs.  Both by bytes
+// plus the fixed cost of a tile, and to fewer warps when there would be less than 4 KB for each.
+void cut_units(const std::vector<FarUnit>& in, const std::vector<FarGroup>& ing, size_t esz,
+               std::vector<StUnit>& out) {
+  const int E = 16 / static_cast<int>(esz);
+  auto z_of = [&](const FarUnit& U) { return (U.flags & 3) == 2 ? ing[U.grp].zdst : U.zout; };  // of the block
+  for (size_t q = 0; q < in.size(); ++q) {
+    const FarUnit& U = in[q];
+    const int32_t z = z_of(U);
+    if (U.ldk > 32 * E) {  // more vectors than lanes: the block in strips of 32 vectors, row by row
+      size_t e = q;
+      while (e + 1 < in.size() && z_of(in[e + 1]) == z) ++e;
+      for (int v = 0; v < U.ldk; v += 32 * E) {
+        const int w = std::min(32 * E, U.ldk - v);
+        for (size_t b = q; b <= e; ++b)
+          for (int c = 0; c < in[b].nc; ++c)
+            out.push_back(StUnit{in[b].voff + static_cast<int64_t>(c) * U.ldk + v, in[b].xc + c, z + v, -1,
+                                 static_cast<int16_t>(w), 1, static_cast<int16_t>(std::max(0, std::min(w, U.k - v))), 0, 0,
+                                 0});
+      }
+      q = e;
+      continue;
+    }
+    int rows = static_cast<int>(ST_TILE / (U.ldk * (int64_t)esz));
+    const int nv = U.ldk / E, round = ST_U * (32 / nv);  // rows of one round of tile_dot
+    if (rows >= round) rows = rows / round * round;
+    for (int a = 0; a < U.nc; a += rows) {
+      const int e = std::min(U.nc, a + rows);
+      out.push_back(StUnit{U.voff + static_cast<int64_t>(a) * U.ldk, U.xc + a, z, -1, static_cast<int16_t>(U.ldk),
+                           static_cast<int16_t>(e - a), static_cast<int16_t>(U.k), 0, 0, 0});
+    }
+  }
+}
+
+// contiguous ranges of `n` things with prefix costs `cost` (n + 1) for `parts` workers
+std::vector<int32_t> deal(const std::vector<double>& cost, int64_t parts) {
+  const int64_t n = static_cast<int64_t>(cost.size()) - 1;
+  std::vector<int32_t> f(parts + 1, 0);
+  int64_t u = 0;
+  for (int64_t w = 0; w <= parts; ++w) {
+    const double target = cost.back() * static_cast<double>(w) / static_cast<double>(parts);
+    while (u < n && cost[u] < target) ++u;
+    f[w] = static_cast<int32_t>(u);
+  }
+  f[parts] = static_cast<int32_t>(n);
+  return f;
+}
+
+// the warp ranges of a unit list; the last unit of a block in each warp writes the block (flags
+// 1) or a partial of a group (flags 2, slots from *ppos)
+std::vector<int32_t> deal_units(std::vector<StUnit>& units, size_t esz, size_t vsz, int64_t parts,
+                                std::vector<FarGroup>& groups, int64_t& ppos) {
+  std::vector<double> cost(units.size() + 1, 0.0);
+  for (size_t u = 0; u < units.size(); ++u)
+    cost[u + 1] = cost[u] + static_cast<double>(units[u].nc) * (units[u].ldk * esz + vsz) + 512.0;
+  for (StUnit& U : units) {
+    const int nv = U.ldk * static_cast<int>(esz) / 16;
+    U.phases = static_cast<uint8_t>(32 / nv);
+    U.magic = 65536 / nv + 1;  // lane / nv = (lane magic) >> 16 for lane < 32, nv <= 32
+  }
+  const std::vector<int32_t> wf = deal(cost, parts);
+  std::vector<int32_t> warp_of(units.size());
+  for (int64_t w = 0; w < parts; ++w)
+    for (int32_t u = wf[w]; u < wf[w + 1]; ++u) warp_of[u] = static_cast<int32_t>(w);
+  for (size_t u = 0; u < units.size();) {
+    size_t e = u;
+    while (e < units.size() && units[e].zout == units[u].zout) ++e;  // block = units [u, e)
+    std::vector<size_t> lasts;
+    for (size_t v = u; v < e; ++v)
+      if (v + 1 == e || warp_of[v + 1] != warp_of[v]) lasts.push_back(v);
+    if (lasts.size() == 1) {
+      units[lasts[0]].flags = 1;
+    } else {
+      const int32_t g = static_cast<int32_t>(groups.size());
+      groups.push_back(FarGroup{static_cast<int32_t>(ppos), static_cast<int32_t>(lasts.size()), units[u].zout,
+                                units[u].k});
+      const int32_t ldk = units[u].ldk;
+      for (size_t c = 0; c < lasts.size(); ++c) {
+        StUnit& L = units[lasts[c]];
+        L.flags = 2;
+        L.grp = g;
+        L.zout = static_cast<int32_t>(ppos + static_cast<int64_t>(c) * ldk);
+      }
+      ppos += static_cast<int64_t>(lasts.size()) * ldk;
+    }
+    u = e;
+  }
+  return wf;
+}
+}  // namespace
+
+void plan_stream(HMatrix& H, const std::vector<FarUnit>& units, const std::vector<FarUnit>& units_h,
+                 const std::vector<FarGroup>& ugroups, const std::vector<int32_t>& seg, const std::vector<int64_t>& ip, const std::vector<int64_t>& hb,
+                 const std::vector<int64_t>& nb, const std::vector<RowItem>& items, cudaStream_t s) {
+  const size_t fsz = H.prec == Prec::F64 ? 8 : H.prec == Prec::MIXED ? 2 : 4, nsz = H.prec == Prec::F64 ? 8 : 4;
+  const int nsm = num_sms(H.device);
+  StreamPlan& S = H.st;
+  // far_z
+  std::vector<StUnit> zu, zh;
+  cut_units(units, ugroups, fsz, zu);
+  cut_units(units_h, ugroups, 2, zh);
+  std::vector<FarGroup> groups;
+  int64_t ppos = 0;
+  auto bytes_of = [](const std::vector<StUnit>& us, size_t esz) {
+    double b = 0.0;
+    for (const StUnit& U : us) b += static_cast<double>(U.nc) * U.ldk * esz;
+    return b;
+  };
+  const int64_t all = static_cast<int64_t>(nsm) * ST_CTAS_PER_SM * ST_WARPS;
+  const int64_t nw = std::max<int64_t>(1, std::min<int64_t>(all, static_cast<int64_t>(bytes_of(zu, fsz) / 4096.0)));
+  const std::vector<int32_t> wf = deal_units(zu, fsz, 8, nw, groups, ppos), wh = deal_units(zh, 2, 8, nw, groups, ppos);
+  SPX_CHECK(ppos < (int64_t(1) << 31), "far-field partial slots exceed 2^31");
+  auto check = [&](const std::vector<StUnit>& us, int64_t pool, size_t esz) {
+    const int E = 16 / static_cast<int>(esz);
+    for (const StUnit& U : us)
+      SPX_CHECK(U.voff % E == 0 && U.ldk % E == 0 && U.nc >= 1 && U.ldk >= U.k && U.ldk <= 32 * E &&
+                    static_cast<int64_t>(U.nc) * U.ldk * (int64_t)esz <= ST_TILE &&
+                    U.voff + static_cast<int64_t>(U.nc) * U.ldk <= pool / (int64_t)esz && U.xc >= 0 &&
+                    U.xc + static_cast<int64_t>(U.nc) <= H.Nb &&
+                    U.zout + static_cast<int64_t>(U.k) <= (U.flags == 2 ? ppos : H.zlen),
+                "stream plan: unit out of range");
+  };
+  check(zu, static_cast<int64_t>(H.far_f.n), fsz);
+  check(zh, static_cast<int64_t>(H.far_h.n), 2);
+  S.zpart_len = ppos;
+  S.nzu = static_cast<int64_t>(zu.size());
+  S.nzh = static_cast<int64_t>(zh.size());
+  S.nwarps = nw;
+  S.zu.upload(zu, s);
+  S.zw.upload(wf, s);
+  S.zh.upload(zh, s);
+  S.zhw.upload(wh, s);
+  S.zgroups.upload(groups, s);
+  S.zcnt.alloc(std::max<size_t>(groups.size(), 1));
+  S.zcnt.zero(s);
+  // rows
+  std::vector<StChunk> ch;
+  std::vector<double> cost(1, 0.0);
+  const int64_t nseg = static_cast<int64_t>(seg.size()) - 1;
+  std::vector<int64_t> seg_c(nseg + 1, 0);
+  for (int64_t g = 0; g < nseg; ++g) {
+    const int nr = seg[g + 1] - seg[g];
+    for (int64_t q = ip[g]; q < ip[g + 1]; ++q) {
+      const int ty = q < hb[g] ? 0 : q < nb[g] ? 1 : 2;
+      const size_t esz = ty == 0 ? fsz : ty == 1 ? 2 : nsz;
+      const int E = 16 / static_cast<int>(esz), ld = (nr + E - 1) / E * E;
+      const RowItem& I = items[q];
+      int rows = static_cast<int>(ST_TILE / (ld * (int64_t)esz));
+      const int round = ST_U * (32 / (ld / E));
+      if (rows >= round) rows = rows / round * round;
+      for (int a = 0; a < I.len; a += rows) {
+        const int e = std::min(I.len, a + rows);
+        ch.push_back(StChunk{I.off + static_cast<int64_t>(a) * ld, I.src + a, static_cast<uint16_t>(e - a),
+                             static_cast<uint8_t>(ld), static_cast<uint8_t>(ty)});
+        cost.push_back(cost.back() + static_cast<double>(e - a) * (ld * esz + 8.0) + 512.0);
+      }
+    }
+    seg_c[g + 1] = static_cast<int64_t>(ch.size());
+  }
+  SPX_CHECK(ch.size() < (size_t(1) << 31), "too many row chunks");
+  for (const StChunk& C : ch) {
+    const int64_t esz = C.type == 0 ? (int64_t)fsz : C.type == 1 ? 2 : (int64_t)nsz;
+    const int64_t pool = static_cast<int64_t>(C.type == 0 ? H.far_f.n : C.type == 1 ? H.far_h.n : H.near_f.n);
+    SPX_CHECK(C.len >= 1 && C.off * esz % 16 == 0 && C.ld * esz % 16 == 0 &&
+                  C.len * C.ld * esz <= ST_TILE && (C.off + static_cast<int64_t>(C.len) * C.ld) * esz <= pool &&
+                  C.src >= 0 && C.src + static_cast<int64_t>(C.len) <= (C.type == 2 ? H.Nb : H.zlen),
+              "stream plan: chunk out of range");
+  }
+  const int nctas = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(static_cast<int64_t>(nsm) * ST_CTAS_PER_SM, static_cast<int64_t>(cost.back() / (4096.0 * ST_WARPS)))));
+  const std::vector<int32_t> cf = deal(cost, nctas);
+  std::vector<StPortion> po;
+  std::vector<int32_t> first(nctas + 1, 0);
+  std::vector<std::vector<int32_t>> of_seg(nseg);  // portions of each segment
+  int64_t g = 0;
+  for (int c = 0; c < nctas; ++c) {
+    int64_t a = cf[c];
+    const int64_t e = cf[c + 1];
+    // segments without chunks (no blocks on their rows) go to the CTA that reaches them
+    while (g < nseg && (a < e || seg_c[g + 1] <= a)) {
+      const int64_t b = std::min<int64_t>(seg_c[g + 1], e);
+      if (b > a || seg_c[g + 1] == seg_c[g]) {
+        of_seg[g].push_back(static_cast<int32_t>(po.size()));
+        po.push_back(StPortion{seg[g], seg[g + 1] - seg[g], static_cast<int32_t>(a), static_cast<int32_t>(b), -1, 0});
+      }
+      a = b;
+      if (seg_c[g + 1] <= a) ++g; else break;
+    }
+    first[c + 1] = static_cast<int32_t>(po.size());
+  }
+  SPX_CHECK(g == nseg, "row plan: not every segment was dealt");
+  std::vector<int2> rg;
+  int32_t slots = 0;
+  for (int64_t q = 0; q < nseg; ++q) {
+    if (of_seg[q].size() < 2) continue;
+    const int32_t id = static_cast<int32_t>(rg.size());
+    rg.push_back(make_int2(slots, static_cast<int>(of_seg[q].size())));
+    for (int32_t p : of_seg[q]) {
+      po[p].grp = id;
+      po[p].slot = slots++;
+    }
+  }
+  S.portions.upload(po, s);
+  S.cta_first.upload(first, s);
+  S.chunks.upload(ch, s);
+  S.rgroups.upload(rg, s);
+  S.rcnt.alloc(std::max<size_t>(rg.size(), 1));
+  S.rcnt.zero(s);
+  S.nslots = slots;
+  S.nctas = nctas;
+  S.ypart.alloc(std::max<int64_t>(slots, 1) * SEG_MAX);
+  S.err.alloc(1);
+  S.err.zero(s);
+  SPX_CUDA(cudaStreamSynchronize(s));  // the host vectors above back the uploads
+}
+
+namespace {
 // FP32 columns kept by a recompressed block under the split packing: the trailing columns go
 // to FP16 when their rounding (relative 2^-11 in U and in V) stays within a tenth of the
 // block's error budget, sqrt(sum_{j>=c} 2 (sigma_j 2^-11)^2) <= 0.1 eps ||A||; rounded up to
@@ -627,11 +872,8 @@ void do_pack(HMatrix& H, cudaStream_t s, bool split = false) {
 
   const int nsm = num_sms(H.device);
   std::vector<FarGroup> groups;
-  int64_t ppos = 0, nw = 0, nwh = 0;
+  int64_t ppos = 0, nw = 0;
   std::vector<int32_t> wf = plan_units(units, sizeof(TF), nsm, nw, groups, ppos);
-  const int32_t g_h0 = static_cast<int32_t>(groups.size());
-  std::vector<int32_t> wfh = plan_units(units_h, 2, nsm, nwh, groups, ppos);
-  (void)g_h0;
   SPX_CHECK(ppos < (int64_t(1) << 31), "far-field partial slots exceed 2^31");
   auto check_units = [&](const std::vector<FarUnit>& us, int64_t cap, int E) {
     for (const FarUnit& U : us)
@@ -643,16 +885,11 @@ void do_pack(HMatrix& H, cudaStream_t s, bool split = false) {
                 "far_z plan: unit out of range");
   };
   check_units(units, fpos, EF);
-  check_units(units_h, hpos, EH);
   H.zpart_len = ppos;
   H.nunits = static_cast<int64_t>(units.size());
   H.nwarps_z = nw;
-  H.nunits_h = static_cast<int64_t>(units_h.size());
-  H.nwarps_z_h = nwh;
   H.units.upload(units, s);
   H.warp_first.upload(wf, s);
-  H.units_h.upload(units_h, s);
-  H.warp_first_h.upload(wfh, s);
   H.groups.upload(groups, s);
   H.gcnt.alloc(std::max<size_t>(groups.size(), 1));
   H.gcnt.zero(s);
@@ -672,56 +909,70 @@ void do_pack(HMatrix& H, cudaStream_t s, bool split = false) {
   H.item_ptr.upload(ip, s);
   H.near_begin.upload(nb, s);
   H.items.upload(items, s);
-  if (H.nunits_h > 0) {
-    H.half_begin.upload(hb, s);
-    H.zscale.upload(zsc, s);
-  } else {
-    H.half_begin.release();
-    H.zscale.release();
-  }
+  if (hpos > 0) H.zscale.upload(zsc, s);
+  else H.zscale.release();
   SPX_CUDA(cudaStreamSynchronize(s));
+  plan_stream(H, units, units_h, groups, seg, ip, hb, nb, items, s);
 }
 
-template <class TF, class TN, class TA, class TX, class TS>
-void launch_apply(HMatrix& H, const TS* src, const int32_t* gidx, TS* dst, const TS* add, TS* yb, TX* xp, TA* z,
+// launch that may start while the kernel before it in the stream finishes (pdl_wait inside)
+template <class... KArgs, class... Args>
+void launch_dependent(void (*k)(KArgs...), unsigned grid, unsigned block, size_t dyn, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = dyn;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  SPX_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...));
+}
+
+template <class TF, class TN, class TA, class TS>
+void launch_apply(HMatrix& H, const TS* src, const int32_t* gidx, TS* dst, const TS* add, TS* yb, TA* xp, TA* z,
                   TA* zpart, cudaStream_t s) {
   const int64_t Nb = H.Nb;
-  k_hgather<TS, TX><<<grid_for(Nb, 256), 256, 0, s>>>(Nb, src, gidx, H.perm.p, xp);
+  StreamPlan& S = H.st;
+  k_hgather<TS, TA><<<grid_for(Nb, 256), 256, 0, s>>>(Nb, src, gidx, H.perm.p, xp);
   SPX_LAUNCH_CHECK();
-  if (H.nunits > 0) {
-    const unsigned ctas = static_cast<unsigned>((H.nwarps_z + Z_WARPS - 1) / Z_WARPS);
-    k_far_z<TF, TA, TX><<<ctas, Z_WARPS * 32, 0, s>>>(H.units.p, H.warp_first.p, static_cast<int>(H.nwarps_z),
-                                                       reinterpret_cast<const TF*>(H.far_f.p), xp, z, zpart,
-                                                       H.groups.p, H.gcnt.p);
-    SPX_LAUNCH_CHECK();
-  }
-  if (H.nunits_h > 0) {  // FP16 trailing columns of the split packing
-    const unsigned ctas = static_cast<unsigned>((H.nwarps_z_h + Z_WARPS - 1) / Z_WARPS);
-    k_far_z<__half, TA, TX><<<ctas, Z_WARPS * 32, 0, s>>>(
-        H.units_h.p, H.warp_first_h.p, static_cast<int>(H.nwarps_z_h), reinterpret_cast<const __half*>(H.far_h.p),
-        xp, z, zpart, H.groups.p, H.gcnt.p);
-    SPX_LAUNCH_CHECK();
-  }
-  const bool half = H.nunits_h > 0;
-  k_rows<TF, TN, TA, TX, TS><<<static_cast<unsigned>(H.nseg), ROWS_WARPS * 32, 0, s>>>(
-      H.seg_start.p, H.item_ptr.p, H.near_begin.p, H.items.p, reinterpret_cast<const TF*>(H.far_f.p),
-      reinterpret_cast<const TN*>(H.near_f.p), z, xp, H.diag_perm.p, H.perm.p, gidx, dst, add, yb,
-      (H.prec != Prec::F64 && sizeof(TA) == sizeof(float)) ? 1 : 0, half ? H.half_begin.p : nullptr,
-      half ? reinterpret_cast<const __half*>(H.far_h.p) : nullptr, half ? H.zscale.p : nullptr);
-  SPX_LAUNCH_CHECK();
+  const unsigned ctas = static_cast<unsigned>(S.nctas), threads = ST_THREADS,
+                 zctas = static_cast<unsigned>((S.nwarps + ST_WARPS - 1) / ST_WARPS);
+  if (S.nzu > 0)
+    launch_dependent(k_far_z<TF, TA>, zctas, threads, 0, s, S.zu.p, S.zw.p, static_cast<int>(S.nwarps),
+                     reinterpret_cast<const TF*>(H.far_f.p), xp, z, zpart, S.zgroups.p, S.zcnt.p,
+                     static_cast<const double*>(nullptr));
+  if (S.nzh > 0)  // FP16 trailing columns of the split packing, scaled back by their singular values
+    launch_dependent(k_far_z<__half, TA>, zctas, threads, 0, s, S.zh.p, S.zhw.p, static_cast<int>(S.nwarps),
+                     reinterpret_cast<const __half*>(H.far_h.p), xp, z, zpart, S.zgroups.p, S.zcnt.p, H.zscale.p);
+  launch_dependent(k_rows<TF, TN, TA, TS>, ctas, threads, 0, s, S.portions.p, S.cta_first.p, S.chunks.p,
+                   reinterpret_cast<const TF*>(H.far_f.p), reinterpret_cast<const TN*>(H.near_f.p),
+                   S.nzh > 0 ? reinterpret_cast<const __half*>(H.far_h.p) : static_cast<const __half*>(nullptr), z, xp, H.diag_perm.p, H.perm.p, gidx, dst, add, yb,
+                   S.rgroups.p, S.rcnt.p, reinterpret_cast<TA*>(S.ypart.p), S.err.p);
 }
 
-template <class TF, class TN, class TA, class TX, class TS>
+template <class TF, class TN, class TA, class TS>
 void do_apply(HMatrix& H, const TS* src, const int32_t* gidx, TS* dst, const TS* add, TS* yb, cudaStream_t s) {
-  const int64_t Nb = H.Nb;
-  if (H.xperm.n < Nb * sizeof(TX)) H.xperm.alloc(Nb * sizeof(TX));
-  if (H.z.n < std::max<int64_t>(H.zlen, 1) * sizeof(TA)) H.z.alloc(std::max<int64_t>(H.zlen, 1) * sizeof(TA));
-  if (H.zpart.n < std::max<int64_t>(H.zpart_len, 1) * sizeof(TA))
-    H.zpart.alloc(std::max<int64_t>(H.zpart_len, 1) * sizeof(TA));
-  launch_apply<TF, TN, TA, TX, TS>(H, src, gidx, dst, add, yb, reinterpret_cast<TX*>(H.xperm.p),
-                                   reinterpret_cast<TA*>(H.z.p), reinterpret_cast<TA*>(H.zpart.p), s);
+  const size_t xb = H.Nb * sizeof(TA), zb = std::max<int64_t>(H.zlen, 1) * sizeof(TA),
+               pb = std::max<int64_t>(H.st.zpart_len, 1) * sizeof(TA);
+  if (H.xperm.n < xb) H.xperm.alloc(xb);
+  if (H.z.n < zb) H.z.alloc(zb);
+  if (H.zpart.n < pb) H.zpart.alloc(pb);
+  launch_apply<TF, TN, TA, TS>(H, src, gidx, dst, add, yb, reinterpret_cast<TA*>(H.xperm.p),
+                               reinterpret_cast<TA*>(H.z.p), reinterpret_cast<TA*>(H.zpart.p), s);
 }
 }  // namespace
+
+int stream_error(HMatrix& H, cudaStream_t s) {
+  if (!H.st.err.n) return 0;
+  int e = 0;
+  SPX_CUDA(cudaMemcpyAsync(&e, H.st.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  SPX_CUDA(cudaMemsetAsync(H.st.err.p, 0, sizeof(int), s));
+  SPX_CUDA(cudaStreamSynchronize(s));
+  return e;
+}
 
 void HMatrix::pack(Prec p, cudaStream_t s) {
   if (p == Prec::SPLIT && !recompressed) recompress(s);  // the split needs SVD-ordered columns
@@ -742,17 +993,17 @@ void HMatrix::apply_gather(const T* src, const int32_t* gidx, T* dst, const T* a
   // FP64 vectors accumulate in FP64 whatever the factor storage; FP32 vectors in FP32
   if (sizeof(T) == sizeof(double)) {
     switch (prec) {
-      case Prec::F64: do_apply<double, double, double, double, T>(*this, src, gidx, dst, add, yb, s); break;
+      case Prec::F64: do_apply<double, double, double, T>(*this, src, gidx, dst, add, yb, s); break;
       case Prec::F32:
-      case Prec::SPLIT: do_apply<float, float, double, double, T>(*this, src, gidx, dst, add, yb, s); break;
-      case Prec::MIXED: do_apply<__nv_bfloat16, float, double, double, T>(*this, src, gidx, dst, add, yb, s); break;
+      case Prec::SPLIT: do_apply<float, float, double, T>(*this, src, gidx, dst, add, yb, s); break;
+      case Prec::MIXED: do_apply<__nv_bfloat16, float, double, T>(*this, src, gidx, dst, add, yb, s); break;
     }
   } else {
     switch (prec) {
-      case Prec::F64: do_apply<double, double, float, float, T>(*this, src, gidx, dst, add, yb, s); break;
+      case Prec::F64: do_apply<double, double, float, T>(*this, src, gidx, dst, add, yb, s); break;
       case Prec::F32:
-      case Prec::SPLIT: do_apply<float, float, float, float, T>(*this, src, gidx, dst, add, yb, s); break;
-      case Prec::MIXED: do_apply<__nv_bfloat16, float, float, float, T>(*this, src, gidx, dst, add, yb, s); break;
+      case Prec::SPLIT: do_apply<float, float, float, T>(*this, src, gidx, dst, add, yb, s); break;
+      case Prec::MIXED: do_apply<__nv_bfloat16, float, float, T>(*this, src, gidx, dst, add, yb, s); break;
     }
   }
 }
@@ -767,8 +1018,7 @@ int64_t HMatrix::device_bytes() const {
   return static_cast<int64_t>(far_f.bytes() + near_f.bytes() + units.bytes() + warp_first.bytes() + groups.bytes() +
                               gcnt.bytes() + seg_start.bytes() + item_ptr.bytes() + near_begin.bytes() +
                               items.bytes() + z.bytes() + zpart.bytes() + xperm.bytes() + diag_perm.bytes() +
-                              perm.bytes() + far_h.bytes() + units_h.bytes() + warp_first_h.bytes() +
-                              half_begin.bytes() + zscale.bytes());
+                              perm.bytes() + far_h.bytes() + zscale.bytes() + st.bytes());
 }
 
 }  // namespace spx
@@ -803,12 +1053,12 @@ void* noalloc_scratch_address() {
   return addr[dev];
 }
 
-template <class TF, class TN, class TA, class TX>
+template <class TF, class TN, class TA>
 void apply_noalloc_impl(HMatrix& H, const double* x, double* y, cudaStream_t s) {
   const int64_t Nb = H.Nb;
-  const size_t xbytes = ((static_cast<size_t>(Nb) * sizeof(TX) + 255) / 256) * 256;
+  const size_t xbytes = ((static_cast<size_t>(Nb) * sizeof(TA) + 255) / 256) * 256;
   const size_t zbytes = ((static_cast<size_t>(std::max<int64_t>(H.zlen, 1)) * sizeof(TA) + 255) / 256) * 256;
-  const size_t pbytes = static_cast<size_t>(std::max<int64_t>(H.zpart_len, 1)) * sizeof(TA);
+  const size_t pbytes = static_cast<size_t>(std::max<int64_t>(H.st.zpart_len, 1)) * sizeof(TA);
   const int64_t cap = g_noalloc_cap.load();
   const size_t limit = cap > 0 ? std::min(kNoAllocScratchBytes, static_cast<size_t>(cap)) : kNoAllocScratchBytes;
   if (xbytes + zbytes + pbytes > limit)
@@ -816,9 +1066,9 @@ void apply_noalloc_impl(HMatrix& H, const double* x, double* y, cudaStream_t s) 
                              "-byte static scratch of spx_hmat_apply_noalloc (needs " +
                              std::to_string(xbytes + zbytes + pbytes) + " bytes); use spx_hmat_apply");
   unsigned char* base = static_cast<unsigned char*>(noalloc_scratch_address());
-  launch_apply<TF, TN, TA, TX, double>(H, x, nullptr, y, nullptr, nullptr, reinterpret_cast<TX*>(base),
-                                       reinterpret_cast<TA*>(base + xbytes),
-                                       reinterpret_cast<TA*>(base + xbytes + zbytes), s);
+  launch_apply<TF, TN, TA, double>(H, x, nullptr, y, nullptr, nullptr, reinterpret_cast<TA*>(base),
+                                   reinterpret_cast<TA*>(base + xbytes), reinterpret_cast<TA*>(base + xbytes + zbytes),
+                                   s);
 }
 
 }  // namespace
@@ -826,10 +1076,10 @@ void apply_noalloc_impl(HMatrix& H, const double* x, double* y, cudaStream_t s) 
 void hmat_apply_noalloc(HMatrix& H, const double* x, double* y, cudaStream_t s) {
   SPX_CHECK(H.packed, "H-matrix is not packed");
   switch (H.prec) {
-    case Prec::F64: apply_noalloc_impl<double, double, double, double>(H, x, y, s); break;
+    case Prec::F64: apply_noalloc_impl<double, double, double>(H, x, y, s); break;
     case Prec::F32:
-    case Prec::SPLIT: apply_noalloc_impl<float, float, double, double>(H, x, y, s); break;
-    case Prec::MIXED: apply_noalloc_impl<__nv_bfloat16, float, double, double>(H, x, y, s); break;
+    case Prec::SPLIT: apply_noalloc_impl<float, float, double>(H, x, y, s); break;
+    case Prec::MIXED: apply_noalloc_impl<__nv_bfloat16, float, double>(H, x, y, s); break;
   }
 }
 

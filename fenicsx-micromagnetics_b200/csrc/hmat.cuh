@@ -83,6 +83,46 @@ struct RowItem {
 
 struct TcPlan;  // hmat_tc.cu
 
+// The stream plan of the single-vector apply (hmat.cu).  StUnit: a tile of a FarUnit, flags 1 / 2 as
+// there, `phases` and `magic` the lane split of its rows.  StChunk: `len` rows of `ld` elements at `off` of a row segment's tile,
+// row q times z[src + q] (type 0: U, 1: FP16 columns of U) or x~[src + q] (type 2: near).
+// StPortion: chunks [c0, c1) of the segment of rows [r0, r0 + nr); grp >= 0: one of several
+// portions of that segment, partial sums at slot `slot`.
+struct alignas(16) StUnit {
+  int64_t voff;
+  int32_t xc, zout, grp;
+  int16_t ldk, nc, k;
+  uint8_t flags, phases;
+  int32_t magic;
+};
+struct alignas(16) StChunk {
+  int64_t off;
+  int32_t src;
+  uint16_t len;
+  uint8_t ld, type;
+};
+struct StPortion {
+  int32_t r0, nr, c0, c1, grp, slot;
+};
+struct StreamPlan {
+  DevBuf<StUnit> zu, zh;           // tiles of V^T (zh: FP16 columns) and the warps' ranges
+  DevBuf<int32_t> zw, zhw;
+  DevBuf<FarGroup> zgroups;        // blocks shared by several warps
+  DevBuf<unsigned int> zcnt;
+  DevBuf<StChunk> chunks;
+  DevBuf<StPortion> portions;
+  DevBuf<int32_t> cta_first;       // [nctas + 1] portions of each CTA
+  DevBuf<int2> rgroups;            // segments shared by several CTAs: first slot, slots
+  DevBuf<unsigned int> rcnt;
+  DevBuf<double> ypart;            // [nslots][64] partial rows
+  DevBuf<int> err;                 // a wait of the apply kernels gave up
+  int64_t nzu = 0, nzh = 0, nwarps = 0, nctas = 0, nslots = 0, zpart_len = 0;
+  size_t bytes() const {
+    return zu.bytes() + zh.bytes() + zw.bytes() + zhw.bytes() + zgroups.bytes() + zcnt.bytes() + chunks.bytes() +
+           portions.bytes() + cta_first.bytes() + rgroups.bytes() + rcnt.bytes() + ypart.bytes() + err.bytes();
+  }
+};
+
 struct RecompressStats {
   int64_t entries_before = 0, entries_after = 0, rewritten = 0;
   double truncation_error_max = 0.0;  // largest truncation error of a block, relative to its norm
@@ -103,24 +143,21 @@ struct HMatrix {
   Prec prec = Prec::F64;
   bool packed = false;
   DevBuf<char> far_f, near_f;     // factor / tile storage in the packed precision
-  DevBuf<FarUnit> units;          // k_far_z work units
-  DevBuf<int32_t> warp_first;     // [nwarps_z + 1] unit range of each k_far_z warp
-  DevBuf<FarGroup> groups;        // far blocks shared by several k_far_z warps
+  DevBuf<FarUnit> units;          // work units of the multi-state far field
+  DevBuf<int32_t> warp_first;     // [nwarps_z + 1] unit range of each of its warps
+  DevBuf<FarGroup> groups;        // far blocks shared by several of them
   DevBuf<unsigned int> gcnt;      // per group: contributors arrived (reset by the last one)
   DevBuf<int32_t> seg_start;      // [nseg + 1] row segments (perm space)
   DevBuf<int64_t> item_ptr;       // [nseg + 1] items of each segment: far ones, then near ones
   DevBuf<int64_t> near_begin;     // [nseg] first near item of each segment
   DevBuf<RowItem> items;
   DevBuf<char> far_h;             // SPLIT: FP16 trailing columns (V^T rows and U tiles)
-  DevBuf<FarUnit> units_h;        // SPLIT: k_far_z units of the FP16 columns
-  DevBuf<int32_t> warp_first_h;
-  DevBuf<int64_t> half_begin;     // SPLIT: [nseg] first FP16 far item of each segment
   DevBuf<double> zscale;          // SPLIT: [zlen] sigma of each FP16 column (1 elsewhere)
-  int64_t nunits_h = 0, nwarps_z_h = 0;
   DevBuf<char> z, zpart;          // far z vectors and partial sums (accumulation type)
   DevBuf<char> xperm;             // x in perm order (vector type)
   int64_t nseg = 0, zlen = 0, zpart_len = 0, n_far = 0, n_near = 0, nunits = 0, nwarps_z = 0;
   int64_t bytes_far = 0, bytes_near = 0;
+  StreamPlan st;                  // single-vector apply; units / items above serve the multi-state one
   std::unique_ptr<HMatrix> tr;    // H^T (same tree; built on first use by transposed())
   DevBuf<double> xmulti, zmulti, zpmulti;  // state-interleaved work vectors of apply_multi
   // far-field GEMMs of apply_multi on the tensor cores for batches of 8 (hmat_tc.cu); null: off
@@ -165,6 +202,15 @@ void hmat_import(HMatrix& H, const BoundaryDev& bd, const HBuildConfig& c, Prec 
 // Block-diagonal concatenation of packed H-matrices (same packing precision) for one apply
 // over all of them (hio.cu); apply-side data only.
 void hmat_merge(const std::vector<const HMatrix*>& parts, HMatrix& M, cudaStream_t s);
+
+// builds H.st from the packing's units, segments and items (host copies; ugroups: the groups that
+// flags-2 units refer to)
+void plan_stream(HMatrix& H, const std::vector<FarUnit>& units, const std::vector<FarUnit>& units_h,
+                 const std::vector<FarGroup>& ugroups, const std::vector<int32_t>& seg, const std::vector<int64_t>& ip,
+                 const std::vector<int64_t>& hb, const std::vector<int64_t>& nb, const std::vector<RowItem>& items,
+                 cudaStream_t s);
+// the timeout code of an apply kernel since the last call, or 0
+int stream_error(HMatrix& H, cudaStream_t s);
 
 // tensor-core far field of the multi-state apply (hmat_tc.cu): tc_build packs the factors
 // (needs the FP64 pools), tc_far_apply returns the far part of Y (perm order, [Nb][8] FP64)

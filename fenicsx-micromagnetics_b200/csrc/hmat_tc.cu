@@ -51,6 +51,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "bulk.cuh"
 #include "hmat.cuh"
 
 namespace spx {
@@ -117,43 +118,9 @@ constexpr int CONV_THREADS = 128;             // warps 8-11
 // + a 32 KB guard after the buffers, so that no descriptor-addressed read can leave the
 // allocation even past the last stage
 constexpr int SMEM_BYTES = NSTAGE * (AST_BYTES + BST_BYTES + BX_BYTES) + 1024 + 32768;
-constexpr long long WAIT_LIMIT = 1ll << 22;  // polls of try_wait before a wait gives up
 static_assert(NDB == 6, "digits6 cuts the B rows");
 static_assert((TM / 8) * 128 * (KS / 16) == AD_BYTES && (NB / 8) * 128 * (KS / 16) == BST_BYTES, "digit tile layouts");
-__device__ __forceinline__ uint32_t su32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(su32(b)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
-  asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(su32(b)),
-               "r"(bytes)
-               : "memory");
-}
-// bounded wait until the phase of parity `par` has completed
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t par) {
-  for (long long it = 0; it < WAIT_LIMIT; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(su32(b)), "r"(par)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   su32(dst)),
-               "l"(src), "r"(bytes), "r"(su32(bar))
-               : "memory");
-}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
