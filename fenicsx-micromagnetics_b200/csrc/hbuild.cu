@@ -32,11 +32,6 @@
 
 namespace spx {
 
-struct FillDesc {
-  int64_t out_off, rows_off, cols_off;
-  int32_t m, n;
-};
-
 // ------------------------------------------------------------------ boundary upload
 void BoundaryDev::create(const double* X, int64_t N, const int32_t* tets, int64_t E) {
   SPX_CUDA(cudaGetDevice(&device));
@@ -71,14 +66,14 @@ void BoundaryDev::fill_block(const int32_t* rows_dev, int64_t m, const int32_t* 
                              double* out, cudaStream_t s) const {
   if (m <= 0 || n <= 0) return;
   FillDesc d{0, 0, 0, static_cast<int32_t>(m), static_cast<int32_t>(n)};
-  const int64_t ntiles = ((m + 127) / 128) * ((n + 31) / 32);
+  const int64_t ntiles = fill_tiles(m, n);
   DevBuf<FillDesc> dd(1);
   DevBuf<int64_t> ts(1);
   int64_t zero = 0;
   dd.upload(&d, 1, s);
   ts.upload(&zero, 1, s);
   launch_fill(dd.p, ts.p, 1, ntiles, rows_dev, cols_dev, Xb.p, tri_lid.p, T.p, inc_ptr.p, inc_tri.p,
-              maxinc, host.Nb, out, s);
+              nullptr, maxinc, host.Nb, out, s);
   SPX_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -135,17 +130,36 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca_update(
   double* R = Apool + d.a_off;
   const double* u = UV + d.u_off + (int64_t)(k - 1) * d.m;
   const double* v = UV + d.v_off + (int64_t)(k - 1) * d.n;
+  // Bound by HBM (16 bytes per entry and step).  Four entries of a thread in flight; row and column
+  // of an entry by stepping (a 64-bit division per entry cost more than its 16 bytes).
   double mv = -1.0, ss = 0.0;
   int64_t mi = INT64_MAX;
-  for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    double r = R[e];
-    if (k > 0) {
-      const int64_t i = e / d.n, j = e - i * d.n;
-      r = __dsub_rn(r, __dmul_rn(u[i], v[j]));
-      R[e] = r;
+  const uint32_t n = static_cast<uint32_t>(d.n);
+  const uint32_t dq = ACA_THREADS / n, dr = ACA_THREADS - dq * n;  // rows and columns of one step
+  const uint32_t f = static_cast<uint32_t>(e0) + threadIdx.x;      // mn < 2^31 (dense block limit)
+  uint32_t i = f / n, j = f - i * n;
+  int64_t e = e0 + threadIdx.x;
+  for (; e < e1; e += 4 * ACA_THREADS) {
+    double r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (e + q * ACA_THREADS < e1) r[q] = R[e + q * ACA_THREADS];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t eq = e + q * ACA_THREADS;
+      if (eq < e1) {
+        if (k > 0) {
+          r[q] = __dsub_rn(r[q], __dmul_rn(u[i], v[j]));
+          R[eq] = r[q];
+        }
+        const double a = fabs(r[q]);
+        if (a > mv) { mv = a; mi = eq; }  // the first of equal entries: eq grows
+        ss += r[q] * r[q];
+        i += dq;
+        j += dr;
+        if (j >= n) { j -= n; ++i; }
+      }
     }
-    better(mv, mi, fabs(r), e);
-    ss += r * r;
   }
   __shared__ double sv[ACA_THREADS / 32], sss[ACA_THREADS / 32];
   __shared__ int64_t si[ACA_THREADS / 32];
@@ -191,7 +205,8 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca_decide(
   if (threadIdx.x == 0) {
     double V = sv[0], S = sss[0];
     int64_t I = si[0];
-    for (int q = 1; q < blockDim.x; ++q) { better(V, I, sv[q], si[q]); S += sss[q]; }
+    const int used = min(static_cast<int>(blockDim.x), d.ntask);  // the others hold nothing
+    for (int q = 1; q < used; ++q) { better(V, I, sv[q], si[q]); S += sss[q]; }
     AcaState s = st[b];
     int go = 1;
     if (s.k == 0) {
@@ -312,9 +327,35 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
   };
 
   const int32_t* pool = perm.p;
-  int* h_active = nullptr;
-  SPX_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_active), sizeof(int)));
+  DevBuf<int32_t> place;  // node -> position in the permutation
+  {
+    std::vector<int32_t> inv(Nb);
+    for (int64_t i = 0; i < Nb; ++i) inv[tree.perm[i]] = static_cast<int32_t>(i);
+    place.upload(inv, s);
+    SPX_CUDA(cudaStreamSynchronize(s));
+  }
   DevBuf<int> d_active(1);
+  // workspace of the batches, kept and grown over the waves (an allocation per buffer and wave took
+  // half of the construction time of a 5,000-row boundary); at most batch_bytes as before
+  DevBuf<double> A, UV;
+  DevBuf<FillDesc> dfd;
+  DevBuf<int64_t> dts;
+  DevBuf<AcaDesc> dad, dupd;
+  DevBuf<AcaState> dst;
+  DevBuf<Partial> dpart;
+  auto room = [](auto& b, int64_t n) {
+    if (static_cast<int64_t>(b.n) < n) {
+      b.release();
+      b.alloc(n);
+    }
+  };
+  auto put = [&](auto& b, const auto& v) {
+    if (b.n < v.size()) {
+      b.release();
+      b.alloc(v.size() + v.size() / 2);
+    }
+    if (!v.empty()) SPX_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, s));
+  };
 
   while (!wave.empty()) {
     stats.waves++;
@@ -342,12 +383,10 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
       int64_t tiles = 0;
       auto flush = [&]() {
         if (fd.empty()) return;
-        DevBuf<FillDesc> dfd;
-        DevBuf<int64_t> dts;
-        dfd.upload(fd, s);
-        dts.upload(ts, s);
+        put(dfd, fd);
+        put(dts, ts);
         launch_fill(dfd.p, dts.p, static_cast<int>(fd.size()), tiles, pool, pool, bd.Xb.p, bd.tri_lid.p,
-                    bd.T.p, bd.inc_ptr.p, bd.inc_tri.p, bd.maxinc, bd.host.Nb, near_g.buf.p, s);
+                    bd.T.p, bd.inc_ptr.p, bd.inc_tri.p, place.p, bd.maxinc, bd.host.Nb, near_g.buf.p, s);
         SPX_CUDA(cudaStreamSynchronize(s));
         fd.clear();
         ts.clear();
@@ -363,7 +402,7 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
         const TreeNode &R = nodes[nearl[q].first], &C = nodes[nearl[q].second];
         ts.push_back(tiles);
         fd.push_back(FillDesc{offs[q], R.start, C.start, R.size(), C.size()});
-        tiles += (int64_t)((R.size() + 127) / 128) * ((C.size() + 31) / 32);
+        tiles += fill_tiles(R.size(), C.size());
         HBlock hb{R.start, R.stop, C.start, C.stop, 0, 0, offs[q], 0, 0.0};
         blocks.push_back(hb);
         stats.dense_blocks++;
@@ -407,29 +446,28 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
                              (int32_t)kmax, early ? 1 : 0, static_cast<int32_t>(ad.size())});
         fd.push_back(FillDesc{a_tot, R.start, C.start, (int32_t)m, (int32_t)n});
         ts.push_back(tiles);
-        tiles += ((m + 127) / 128) * ((n + 31) / 32);
+        tiles += fill_tiles(m, n);
         tasks += ad.back().ntask;
         a_tot += mn;
         uv_tot += kcap * (m + n);
         ++q1;
       }
       const int nb = static_cast<int>(ad.size());
-      DevBuf<double> A(a_tot), UV(std::max<int64_t>(uv_tot, 1));
-      DevBuf<FillDesc> dfd;
-      DevBuf<int64_t> dts;
-      dfd.upload(fd, s);
-      dts.upload(ts, s);
-      launch_fill(dfd.p, dts.p, nb, tiles, pool, pool, bd.Xb.p, bd.tri_lid.p, bd.T.p, bd.inc_ptr.p,
-                  bd.inc_tri.p, bd.maxinc, bd.host.Nb, A.p, s);
-      stats.block_entry_evaluations += a_tot;
-      DevBuf<AcaDesc> dad, dupd;
-      dad.upload(ad, s);
-      DevBuf<AcaState> dst(nb);
-      {
-        std::vector<AcaState> h0(nb, AcaState{0, 0, 0, 0, 0.0, 1.0});
-        dst.upload(h0, s);
+      if (static_cast<int64_t>(A.n) < a_tot || static_cast<int64_t>(UV.n) < uv_tot) {
+        A.release();  // together: a batch may be all factors or all entries
+        UV.release();
+        A.alloc(a_tot);
+        UV.alloc(std::max<int64_t>(uv_tot, 1));
       }
-      DevBuf<Partial> dpart(std::max<int64_t>(tasks, 1));
+      put(dfd, fd);
+      put(dts, ts);
+      launch_fill(dfd.p, dts.p, nb, tiles, pool, pool, bd.Xb.p, bd.tri_lid.p, bd.T.p, bd.inc_ptr.p,
+                  bd.inc_tri.p, place.p, bd.maxinc, bd.host.Nb, A.p, s);
+      stats.block_entry_evaluations += a_tot;
+      put(dad, ad);
+      const std::vector<AcaState> h0(nb, AcaState{0, 0, 0, 0, 0.0, 1.0});
+      put(dst, h0);
+      room(dpart, std::max<int64_t>(tasks, 1));
       int active = nb;
       SPX_CUDA(cudaMemcpyAsync(d_active.p, &active, sizeof(int), cudaMemcpyHostToDevice, s));
       // update launch list (compacted to the active blocks as they finish)
@@ -450,9 +488,9 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
         ++step;
         stats.aca_steps++;
         if (step % check_every == 0 || step >= max_steps) {
-          SPX_CUDA(cudaMemcpyAsync(h_active, d_active.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+          int act = 0;
+          SPX_CUDA(cudaMemcpyAsync(&act, d_active.p, sizeof(int), cudaMemcpyDeviceToHost, s));
           SPX_CUDA(cudaStreamSynchronize(s));
-          const int act = *h_active;
           if (act == 0) break;
           if (step >= max_steps) throw Error(ERR_INTERNAL, "ACA batch did not finish within kmax steps");
           if (2 * act < n_upd) {
@@ -468,7 +506,7 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
                 t0 += d.ntask;
                 sub.push_back(d);
               }
-            dupd.upload(sub, s);
+            put(dupd, sub);
             upd = dupd.p;
             n_upd = static_cast<int>(sub.size());
             upd_tasks = t0;
@@ -520,7 +558,7 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
           // A now holds the residual: refill the original entries into the near pool
           rts.push_back(rt);
           rf.push_back(FillDesc{dn[bq], fd[bq].rows_off, fd[bq].cols_off, fd[bq].m, fd[bq].n});
-          rt += (int64_t)((fd[bq].m + 127) / 128) * ((fd[bq].n + 31) / 32);
+          rt += fill_tiles(fd[bq].m, fd[bq].n);
           blocks.push_back(HBlock{R.start, R.stop, C.start, C.stop, 0, 0, dn[bq], 0, st.rel});
           stats.dense_blocks++;
           stats.rejected_low_rank_blocks++;
@@ -533,12 +571,10 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
         }
       }
       if (!rf.empty()) {
-        DevBuf<FillDesc> drf;
-        DevBuf<int64_t> drts;
-        drf.upload(rf, s);
-        drts.upload(rts, s);
-        launch_fill(drf.p, drts.p, static_cast<int>(rf.size()), rt, pool, pool, bd.Xb.p, bd.tri_lid.p,
-                    bd.T.p, bd.inc_ptr.p, bd.inc_tri.p, bd.maxinc, bd.host.Nb, near_g.buf.p, s);
+        put(dfd, rf);
+        put(dts, rts);
+        launch_fill(dfd.p, dts.p, static_cast<int>(rf.size()), rt, pool, pool, bd.Xb.p, bd.tri_lid.p,
+                    bd.T.p, bd.inc_ptr.p, bd.inc_tri.p, place.p, bd.maxinc, bd.host.Nb, near_g.buf.p, s);
       }
       run_copy_jobs(jobs, s);
       SPX_CUDA(cudaStreamSynchronize(s));
@@ -546,7 +582,9 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
     }
     wave.swap(next);
   }
-  cudaFreeHost(h_active);
+  A.release();
+  UV.release();
+  dpart.release();
   far_pool64 = std::move(far_g.buf);
   near_pool64 = std::move(near_g.buf);
   stats.n_far = stats.low_rank_blocks;

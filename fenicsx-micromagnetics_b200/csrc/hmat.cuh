@@ -7,11 +7,21 @@
 
 namespace spx {
 
-struct FillDesc;
+struct FillDesc {
+  int64_t out_off;   // offset of the block in the output pool (row-major m x n)
+  int64_t rows_off;  // offset into rows pool
+  int64_t cols_off;  // offset into cols pool
+  int32_t m, n;
+};
+constexpr int FILL_TR = 32, FILL_TC = 32;  // rows and columns of a fill tile
+inline int64_t fill_tiles(int64_t m, int64_t n) {
+  return ((m + FILL_TR - 1) / FILL_TR) * ((n + FILL_TC - 1) / FILL_TC);
+}
+// place: position of every boundary node in cols_pool when that is a permutation of them, or null
 void launch_fill(const FillDesc* d_blocks, const int64_t* d_tile_start, int nb, int64_t ntiles,
                  const int32_t* rows_pool, const int32_t* cols_pool, const double* Xb,
                  const int32_t* tri_lid, const double* T, const int32_t* inc_ptr,
-                 const int32_t* inc_tri, int maxinc, int64_t Nb, double* out, cudaStream_t s);
+                 const int32_t* inc_tri, const int32_t* place, int maxinc, int64_t Nb, double* out, cudaStream_t s);
 void launch_lindholm_pairs(int64_t P, const double* x0, const int32_t* tri, const double* T, int64_t Nt, double* w,
                            cudaStream_t s);
 void launch_add_diag(int64_t Nb, const double* omega_sum, double* B, cudaStream_t s);

@@ -4,17 +4,20 @@
 // (solid angle via atan2, edge logs via log1p with the 1e-300 floor, opposite-edge
 // convention) and of the block fill of lindholm_hmatrix_gpu/entry_provider.py:41-117.
 //
-// Fill design.  A CTA owns a tile of TR=128 block rows x TC=32 block columns.  Its
-// first 32 threads build the list of triangles incident to the tile's columns (each
-// triangle kept once, by its lowest in-tile column, in a fixed order so results are
-// deterministic), then every thread (one per row) walks that list, evaluates the three
-// weights once per (row, triangle) and adds them to its private row of a shared-memory
-// accumulator.  Triangles incident to the row vertex are skipped (incident_policy
+// Fill design.  A warp owns a tile of TR=32 block rows x TC=32 block columns.  Its threads
+// build the list of triangles incident to the tile's columns (each triangle kept once, by
+// its lowest in-tile column, in a fixed order so results are deterministic; a triangle's
+// columns found by the node's place in the permutation where the columns are a stretch of
+// it), then every thread (one per row) walks that list, evaluates the three weights once
+// per (row, triangle) and adds them to its private row of a shared-memory accumulator.
+// Bound by FP64 arithmetic (about 500 operations a weight triple).  Rows of a leaf block are
+// about 40: tiles of 128 rows left two thirds of the threads idle there, and the search of
+// the column list by compares took a quarter of the time.  Triangles incident to the row vertex are skipped (incident_policy
 // "skip", gpu/fields/Demag_Lindholm.py:87-96).  The tile is written back row-major with
 // consecutive threads on consecutive columns.  No atomics.
 #include <cmath>
 
-#include "spx_internal.cuh"
+#include "hmat.cuh"
 
 namespace spx {
 
@@ -73,23 +76,14 @@ __global__ void k_lindholm_pairs(int64_t P, const double* __restrict__ x0, const
   w[3 * k + 2] = c;
 }
 
-struct FillDesc {
-  int64_t out_off;   // offset of the block in the output pool (row-major m x n)
-  int64_t rows_off;  // offset into rows pool
-  int64_t cols_off;  // offset into cols pool
-  int32_t m, n;
-};
-
-constexpr int FILL_TR = 128;
-constexpr int FILL_TC = 32;
-
 // tile_start[b] = first task of block b (prefix sum of ceil(m/TR)*ceil(n/TC)); nb blocks
 __global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
     const FillDesc* __restrict__ blocks, const int64_t* __restrict__ tile_start, int nb,
     const int32_t* __restrict__ rows_pool, const int32_t* __restrict__ cols_pool,
     const double* __restrict__ Xb, const int32_t* __restrict__ tri_lid,
     const double* __restrict__ T, const int32_t* __restrict__ inc_ptr,
-    const int32_t* __restrict__ inc_tri, int maxinc, int64_t Nb, double* __restrict__ out) {
+    const int32_t* __restrict__ inc_tri, const int32_t* __restrict__ place, int maxinc, int64_t Nb,
+    double* __restrict__ out) {
   extern __shared__ double smem[];
   double* acc = smem;                                                       // [TR][TC+1]
   int32_t* scol = reinterpret_cast<int32_t*>(acc + FILL_TR * (FILL_TC + 1));  // [TC]
@@ -129,8 +123,13 @@ __global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
         for (int v = 0; v < 3; ++v) {
           const int32_t gv = tri_lid[3 * (int64_t)t + v];
           slot[v] = -1;
-          for (int c = 0; c < tc; ++c)
-            if (scol[c] == gv) { slot[v] = c; break; }
+          if (place) {  // cols_pool[place[gv]] = gv
+            const int64_t c = place[gv] - (bd.cols_off + col0);
+            if (c >= 0 && c < tc) slot[v] = static_cast<int>(c);
+          } else {
+            for (int c = 0; c < tc; ++c)
+              if (scol[c] == gv) { slot[v] = c; break; }
+          }
           if (slot[v] >= 0 && slot[v] < first) first = slot[v];
         }
         if (first == tid && cnt < maxinc) {
@@ -187,7 +186,7 @@ size_t fill_smem_bytes(int maxinc) {
 void launch_fill(const FillDesc* d_blocks, const int64_t* d_tile_start, int nb, int64_t ntiles,
                  const int32_t* rows_pool, const int32_t* cols_pool, const double* Xb,
                  const int32_t* tri_lid, const double* T, const int32_t* inc_ptr,
-                 const int32_t* inc_tri, int maxinc, int64_t Nb, double* out, cudaStream_t s) {
+                 const int32_t* inc_tri, const int32_t* place, int maxinc, int64_t Nb, double* out, cudaStream_t s) {
   if (ntiles <= 0) return;
   const size_t smem = fill_smem_bytes(maxinc);
   static bool attr_set = false;
@@ -199,7 +198,8 @@ void launch_fill(const FillDesc* d_blocks, const int64_t* d_tile_start, int nb, 
   SPX_CHECK(ntiles < (1ll << 31), "fill launch too large; split the batch");
   {
     k_fill_tiles<<<static_cast<unsigned>(ntiles), FILL_TR, smem, s>>>(
-        d_blocks, d_tile_start, nb, rows_pool, cols_pool, Xb, tri_lid, T, inc_ptr, inc_tri, maxinc, Nb, out);
+        d_blocks, d_tile_start, nb, rows_pool, cols_pool, Xb, tri_lid, T, inc_ptr, inc_tri, place, maxinc, Nb,
+        out);
     SPX_LAUNCH_CHECK();
   }
 }
