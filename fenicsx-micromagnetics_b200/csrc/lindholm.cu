@@ -11,8 +11,9 @@
 // it), then every thread (one per row) walks that list, evaluates the three weights once
 // per (row, triangle) and adds them to its private row of a shared-memory accumulator.
 // Bound by FP64 arithmetic (about 500 operations a weight triple).  Rows of a leaf block are
-// about 40: tiles of 128 rows left two thirds of the threads idle there, and the search of
-// the column list by compares took a quarter of the time.  Triangles incident to the row vertex are skipped (incident_policy
+// about 40, so tiles of 128 rows left two thirds of the threads idle there.  With the lookup in
+// place of a search by compares: 5.8 -> 5.0 ms (4,994 rows), 55.8 -> 49.9 ms (20,802 rows), both
+// changes together.  Triangles incident to the row vertex are skipped (incident_policy
 // "skip", gpu/fields/Demag_Lindholm.py:87-96).  The tile is written back row-major with
 // consecutive threads on consecutive columns.  No atomics.
 #include <cmath>
