@@ -60,9 +60,14 @@ __device__ __forceinline__ void vec_elems(const double2& v, double e[2]) { e[0] 
 
 // CTA per tile of up to TILE_ROWS rows of one dense sample: the sample's boundary vector x
 // is staged in shared memory (FP64, nb_s <= dense_max_nb entries), then each warp streams
-// its rows of B_s as 16-byte vectors (rows padded to 16 bytes, four vectors in flight per
-// lane):  g = B_s[i, :] . x,  gB[b0_s + i] = g,  phi[bverts[b0_s + i]] = u1 + g.
+// two rows of B_s at a time as 16-byte vectors (rows padded to 16 bytes, four vectors of each
+// row in flight per lane, the last batch of a row included):
+//   g = B_s[i, :] . x,  gB[b0_s + i] = g,  phi[bverts[b0_s + i]] = u1 + g.
+// Bound by HBM: 49 blocks of up to 3,990 rows, FP32 (1.28 GB) 250 -> 196 us = 6.5 TB/s.  One row
+// with a serial remainder left 20% of it; rows x vectors 1x5 to 4x3 lie within 195..204 us, 8x1
+// takes 311.
 constexpr int TILE_ROWS = 64;
+constexpr int GEMV_ROWS = 2, GEMV_VECS = 4;
 template <class TV, class TM>
 __global__ void __launch_bounds__(256) k_block_gemv(const int32_t* __restrict__ tiles, const int64_t* __restrict__ b0,
                                                     const int64_t* __restrict__ nbv, const int64_t* __restrict__ off,
@@ -75,41 +80,59 @@ __global__ void __launch_bounds__(256) k_block_gemv(const int32_t* __restrict__ 
   const int q = tiles[2 * blockIdx.x], i0 = tiles[2 * blockIdx.x + 1];
   const int64_t n = nbv[q], base = b0[q];
   const int64_t nv = block_ld<TM>(n) / E;
-  for (int64_t j = threadIdx.x; j < nv * E; j += blockDim.x) xs[j] = j < n ? static_cast<double>(xb[base + j]) : 0.0;
+  // entries of x by pairs: pair p of vector v at 2 (p nv + v), so a warp's 16-byte reads of one
+  // pair are consecutive
+  for (int64_t j = threadIdx.x; j < nv * E; j += blockDim.x) {
+    const int64_t v = j / E, u = j % E;
+    xs[2 * ((u >> 1) * nv + v) + (u & 1)] = j < n ? static_cast<double>(xb[base + j]) : 0.0;
+  }
   __syncthreads();
+  const double2* x2 = reinterpret_cast<const double2*>(xs);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int64_t i1 = std::min<int64_t>(n, i0 + TILE_ROWS);
-  for (int64_t i = i0 + wid; i < i1; i += nwarp) {
-    const VT* row = reinterpret_cast<const VT*>(pool + off[q] + i * nv * E);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    int64_t v = lane;
-    for (; v + 96 < nv; v += 128) {
-      VT w[4];
+  for (int64_t i = i0 + wid; i < i1; i += GEMV_ROWS * nwarp) {
+    const VT* row[GEMV_ROWS];  // a row past the end repeats the first and is not stored
 #pragma unroll
-      for (int t = 0; t < 4; ++t) w[t] = __ldcs(row + v + 32 * t);
+    for (int r = 0; r < GEMV_ROWS; ++r)
+      row[r] = reinterpret_cast<const VT*>(pool + off[q] + (i + r * nwarp < i1 ? i + r * nwarp : i) * nv * E);
+    double acc[GEMV_ROWS] = {};
+    for (int64_t v = lane; v < nv; v += 32 * GEMV_VECS) {
+      VT w[GEMV_VECS][GEMV_ROWS];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        double e[E];
-        vec_elems(w[t], e);
-        const double* xv = xs + (v + 32 * t) * E;  // padding entries of B are zero
+      for (int t = 0; t < GEMV_VECS; ++t)
+        if (v + 32 * t < nv) {
 #pragma unroll
-        for (int u = 0; u < E; ++u) acc[t] += e[u] * xv[u];
+          for (int r = 0; r < GEMV_ROWS; ++r) w[t][r] = __ldcs(row[r] + v + 32 * t);
+        }
+#pragma unroll
+      for (int t = 0; t < GEMV_VECS; ++t)
+        if (v + 32 * t < nv) {
+          double x[E];
+#pragma unroll
+          for (int p = 0; p < E / 2; ++p) {
+            const double2 xp = x2[p * nv + v + 32 * t];
+            x[2 * p] = xp.x;
+            x[2 * p + 1] = xp.y;
+          }
+#pragma unroll
+          for (int r = 0; r < GEMV_ROWS; ++r) {
+            double e[E];
+            vec_elems(w[t][r], e);
+#pragma unroll
+            for (int u = 0; u < E; ++u) acc[r] += e[u] * x[u];  // padding: zero times zero
+          }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < GEMV_ROWS; ++r) {
+      const double g = warp_sum(acc[r]);
+      if (lane == 0 && i + r * nwarp < i1) {
+        const TV y = static_cast<TV>(g);
+        const int64_t k = base + i + r * nwarp;
+        gB[k] = y;
+        const int32_t vtx = bverts[k];
+        phi[vtx] = u1[vtx] + y;
       }
-    }
-    for (; v < nv; v += 32) {
-      double e[E];
-      vec_elems(__ldcs(row + v), e);
-      const int64_t c = v * E;
-#pragma unroll
-      for (int u = 0; u < E; ++u)
-        if (c + u < n) acc[0] += e[u] * xs[c + u];
-    }
-    const double g = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
-    if (lane == 0) {
-      const TV y = static_cast<TV>(g);
-      gB[base + i] = y;
-      const int32_t vtx = bverts[base + i];
-      phi[vtx] = u1[vtx] + y;
     }
   }
 }
