@@ -582,8 +582,11 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
       if (gm <= itol * itol * g0 || total >= P.maxit || !(gm > 0.0) || !(dl > 0.0)) break;
       const double beta = gm * ginv;  // 0 on the first step
       den = dl - beta * beta * den;
+      if (!(den > 0.0)) break;  // lost to rounding: the next refinement starts from the true residual
       bt = static_cast<TM>(beta);
-      a = static_cast<TM>(gm) / static_cast<TM>(den);
+      // the quotient in FP64, then rounded: gm and den are squares of the residual's norm and leave
+      // the range of FP32 (1e-38) long before the residual does
+      a = static_cast<TM>(gm / den);
       ginv = 1.0 / gm;
     }
     CG_ROWS_BEGIN
