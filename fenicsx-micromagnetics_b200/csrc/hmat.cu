@@ -465,7 +465,9 @@ void run_pack_jobs(const std::vector<PackJob>& jobs, const double* pool, const d
 
 // far_z units dealt to warps in contiguous ranges of about equal cost; the last unit of a
 // block in each warp writes the block (flags 1), or contributes partials to a group (flags 2)
-// whose slots start at *ppos.  Returns the warp ranges.
+// whose slots start at *ppos.  Every unit of a block with more vectors per row than a warp has
+// lanes is a contribution of its own (k_far_z_multi goes over its rows in strips of 32 vectors).
+// Returns the warp ranges.
 std::vector<int32_t> plan_units(std::vector<FarUnit>& units, size_t elem_bytes, int nsm, int64_t& nw_out,
                                 std::vector<FarGroup>& groups, int64_t& ppos) {
   const int64_t nw = std::max<int64_t>(1, std::min<int64_t>(static_cast<int64_t>(nsm) * Z_CTAS_PER_SM * Z_WARPS,
@@ -492,9 +494,10 @@ std::vector<int32_t> plan_units(std::vector<FarUnit>& units, size_t elem_bytes, 
   while (u < units.size()) {
     size_t e = u;
     while (e < units.size() && units[e].zout == units[u].zout) ++e;  // block = units [u, e)
+    const bool wide = static_cast<int64_t>(units[u].ldk) * static_cast<int64_t>(elem_bytes) > 32 * 16;
     std::vector<size_t> lasts;
     for (size_t v = u; v < e; ++v)
-      if (v + 1 == e || warp_of[v + 1] != warp_of[v]) lasts.push_back(v);
+      if (wide || v + 1 == e || warp_of[v + 1] != warp_of[v]) lasts.push_back(v);
     if (lasts.size() == 1) {
       units[lasts[0]].flags = 1;
     } else {

@@ -98,23 +98,40 @@ __global__ void __launch_bounds__(MZ_WARPS * 32, W16<TF>::E * R >= 64 ? 1 : 2)
       pf_l2(F + Nx.voff, static_cast<uint32_t>(Nx.nc) * Nx.ldk * sizeof(TF));
     }
     const int nvq = U.ldk / E;
-    const int lg = lg32(nvq);
-    const int G = 1 << lg, P = 32 >> lg;
-    const int vl = lane & (G - 1), ph = lane >> lg;
-    if (vl < nvq) {
-      const VT* tile = reinterpret_cast<const VT*>(F + U.voff) + vl;
-      const double* x = xm + static_cast<int64_t>(U.xc) * R;
-      int c = ph;
-      constexpr int UF = InFlight<E, R>::UF;
-      for (; c + (UF - 1) * P < U.nc; c += UF * P) {  // UF factor vectors in flight
-        VT w[UF];
+    const int fl = U.flags & 3;
+    // strips of 32 vectors of the rows: one, unless a row has more vectors than the warp has lanes;
+    // such a unit ends its contribution (plan_units), so the accumulators serve one strip at a time
+    for (int s0 = 0; s0 < nvq; s0 += 32) {
+      const int nv = min(32, nvq - s0);
+      const int lg = lg32(nv);
+      const int G = 1 << lg, P = 32 >> lg;
+      const int vl = lane & (G - 1), ph = lane >> lg;
+      if (vl < nv) {
+        const VT* tile = reinterpret_cast<const VT*>(F + U.voff) + s0 + vl;
+        const double* x = xm + static_cast<int64_t>(U.xc) * R;
+        int c = ph;
+        constexpr int UF = InFlight<E, R>::UF;
+        for (; c + (UF - 1) * P < U.nc; c += UF * P) {  // UF factor vectors in flight
+          VT w[UF];
 #pragma unroll
-        for (int u = 0; u < UF; ++u) w[u] = tile[static_cast<int64_t>(c + u * P) * nvq];
+          for (int u = 0; u < UF; ++u) w[u] = tile[static_cast<int64_t>(c + u * P) * nvq];
 #pragma unroll
-        for (int u = 0; u < UF; ++u) {
+          for (int u = 0; u < UF; ++u) {
+            double e[E];
+            elems(w[u], e);
+            const double* xr = x + static_cast<int64_t>(c + u * P) * R;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              const double a = xr[r];
+#pragma unroll
+              for (int t = 0; t < E; ++t) acc[t][r] += e[t] * a;
+            }
+          }
+        }
+        for (; c < U.nc; c += P) {
           double e[E];
-          elems(w[u], e);
-          const double* xr = x + static_cast<int64_t>(c + u * P) * R;
+          elems(tile[static_cast<int64_t>(c) * nvq], e);
+          const double* xr = x + static_cast<int64_t>(c) * R;
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             const double a = xr[r];
@@ -123,39 +140,27 @@ __global__ void __launch_bounds__(MZ_WARPS * 32, W16<TF>::E * R >= 64 ? 1 : 2)
           }
         }
       }
-      for (; c < U.nc; c += P) {
-        double e[E];
-        elems(tile[static_cast<int64_t>(c) * nvq], e);
-        const double* xr = x + static_cast<int64_t>(c) * R;
+      if (fl == 0) break;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const double a = xr[r];
+      for (int t = 0; t < E; ++t)
 #pragma unroll
-          for (int t = 0; t < E; ++t) acc[t][r] += e[t] * a;
+        for (int r = 0; r < R; ++r)
+          for (int o = G; o < 32; o <<= 1) acc[t][r] += __shfl_xor_sync(0xffffffffu, acc[t][r], o);
+      double* out = fl == 1 ? z : zpart;
+      if (ph == 0 && vl < nv) {
+#pragma unroll
+        for (int t = 0; t < E; ++t) {
+          const int q = (s0 + vl) * E + t;
+          if (q < U.k)
+#pragma unroll
+            for (int r = 0; r < R; ++r) out[(static_cast<int64_t>(U.zout) + q) * R + r] = acc[t][r];
         }
       }
+#pragma unroll
+      for (int t = 0; t < E; ++t)
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[t][r] = 0.0;
     }
-    const int fl = U.flags & 3;
-    if (fl == 0) continue;
-#pragma unroll
-    for (int t = 0; t < E; ++t)
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        for (int o = G; o < 32; o <<= 1) acc[t][r] += __shfl_xor_sync(0xffffffffu, acc[t][r], o);
-    double* out = fl == 1 ? z : zpart;
-    if (ph == 0 && vl < nvq) {
-#pragma unroll
-      for (int t = 0; t < E; ++t) {
-        const int q = vl * E + t;
-        if (q < U.k)
-#pragma unroll
-          for (int r = 0; r < R; ++r) out[(static_cast<int64_t>(U.zout) + q) * R + r] = acc[t][r];
-      }
-    }
-#pragma unroll
-    for (int t = 0; t < E; ++t)
-#pragma unroll
-      for (int r = 0; r < R; ++r) acc[t][r] = 0.0;
     if (fl == 2) {  // block shared between warps: the last contributor sums the partials in order
       __threadfence();
       __syncwarp();
