@@ -416,9 +416,10 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
   double bb = 0.0, rho = 0.0, rho0 = -1.0, tol2 = 0.0;
   bool zero = !P.warm;  // y = 0
   int total = 0, outers = 0;
-  for (int outer = 0; outer < P.max_outer; ++outer) {
+  for (int outer = 0;; ++outer) {
     ++outers;
-    // true residual in FP64 (and, the first time, the right-hand side); start of the inner solve
+    // true residual in FP64 (and, the first time, the right-hand side); start of the inner solve.
+    // After the last of max_outer inner solves too: the residual reported is that of the solution.
     {
       double rh = 0.0, b2 = 0.0;
       CG_ROWS_BEGIN
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
     }
     zero = false;
     if (rho0 < 0.0) rho0 = rho;
-    if (rho <= tol2 || total >= P.maxit) break;
+    if (rho <= tol2 || total >= P.maxit || outer == P.max_outer) break;
     // reduce the residual only as far as the target needs (with a 0.3 margin), at most
     // by inner_rtol per refinement step (the inner solve's reliable range)
     const double need = 0.3 * sqrt(tol2 / rho);
@@ -901,7 +902,6 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
     if (h_err) throw Error(ERR_TIMEOUT, "CG grid barrier timed out");
     out.iterations = h_it;
     out.rel_residual = h_res;
-    out.converged = (h_res <= rtol || h_it < maxit) ? 1 : 0;
   }
   return out;
 }

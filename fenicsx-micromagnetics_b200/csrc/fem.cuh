@@ -22,7 +22,6 @@ namespace spx {
 struct CgStats {
   int64_t iterations = 0;
   double rel_residual = 0.0;
-  int converged = 0;
 };
 
 // Per-category CUDA-event timing of the demag/LLG pipeline (enabled on demand; events

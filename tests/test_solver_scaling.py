@@ -126,3 +126,25 @@ def test_field_is_linear_in_the_magnetisation(dims, precision, pc):
             assert float(field(d, torch.zeros_like(m)).abs().max()) == 0.0
         else:
             assert _rel(field(d, m * 2.0 ** e) * 2.0 ** -e, ref) < tol, e
+
+
+# The u2 solve of the last stage (the first in reverse) starts 3e62 times too large, and a refinement
+# gains 7 digits in FP64: the last of the ten refinements reaches the tolerance (3e62 1e-70 = 3e-8), the
+# ninth does not (3e62 1e-63 = 0.3, less at most CG's last step per refinement).  The residual that is
+# reported has to be that of the solution that is returned.
+@pytest.mark.parametrize("dims", MESHES)
+def test_reported_residual_is_that_of_the_solution(dims):
+    import torch
+    X, T = _mesh(dims)
+    rtol = 1e-6
+    hef = _field(X, T, "f64", "extrapolate", rtol)
+    m = _unit(X.shape[0], 4)
+    lam = torch.as_tensor(np.random.default_rng(2).normal(size=m.numel()), device="cuda")
+
+    def reported():
+        return hef.demag_field.solver_counters()["u2"]["final_rel_residual_sum"]
+
+    _step_vjp(hef, m, lam * 3e62)
+    before = reported()
+    _step_vjp(hef, m, lam)
+    assert reported() - before <= 4 * rtol  # four stages
