@@ -890,19 +890,19 @@ __device__ __forceinline__ void post_c(const AmgLevelDev& L, const AmgResident& 
 // (d, u) of the PCG
 template <bool TOP>
 __device__ __forceinline__ void post_d(const AmgLevelDev& L, const AmgResident& R, const LvlBlock& B, const double* r64,
-                                       double& rz, double& wz) {
+                                       const double* diag, double& rz, double& wz) {
   const float rho0 = 1.0f / L.sigma, rho1 = 1.0f / (2.0f * L.sigma - rho0);
   const float it = 1.0f / L.theta, c0 = rho1 * rho0 * it, c1 = 2.0f * rho1 / L.delta;
   BLOCK_ROWS_BEGIN(B, L.n)
     const float di = L.dinv[i], r0 = L.r[i], x2 = L.x2[i];
-    const double rd = TOP ? r64[i] : 0.0;
+    const double rd = TOP ? r64[i] : 0.0, dg = TOP ? diag[i] : 0.0;
     const float t = block_dot(L, R, B, k, lane, L.r) * it;
     const float r1 = r0 - di * t;
     const float z = x2 + (c0 * r0 + c1 * r1);
     L.x[i] = z;
     if (TOP) {
       rz += rd * static_cast<double>(z);
-      wz += static_cast<double>(z / di);
+      wz += dg * static_cast<double>(z);
     }
   BLOCK_ROWS_END
 }
@@ -1037,10 +1037,10 @@ __device__ __forceinline__ bool vcycle(const PcgParams<TV>& P, PcgShared& S, int
     if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     pcg_mark(tm, ph++, P.timing);
     if (l == 0) {
-      post_d<true>(L, P.R[l], S.blk[l], P.r, rz, wz);
+      post_d<true>(L, P.R[l], S.blk[l], P.r, P.diag, rz, wz);
       if (!sync_sum(P, S, flip, rz, wz)) return false;
     } else {
-      post_d<false>(L, P.R[l], S.blk[l], nullptr, rz, wz);
+      post_d<false>(L, P.R[l], S.blk[l], nullptr, nullptr, rz, wz);
       if (!grid_barrier(cnt, nullptr, nb, P.err)) return false;
     }
     pcg_mark(tm, ph++, P.timing);
