@@ -953,8 +953,7 @@ int spx_hmat_tc_status(spx_hmat hm, int32_t* status) {
   API_BEGIN
   REQUIRE(hm); REQUIRE(status);
   HMatrix& H = hm->h();
-  const int e = tc_error(H, 0), f = stream_error(H, 0);
-  *status = e ? e : f;
+  *status = tc_error(H, 0);
   API_END
 }
 

@@ -125,11 +125,10 @@ struct StreamPlan {
   DevBuf<int2> rgroups;            // segments shared by several CTAs: first slot, slots
   DevBuf<unsigned int> rcnt;
   DevBuf<double> ypart;            // [nslots][64] partial rows
-  DevBuf<int> err;                 // a wait of the apply kernels gave up
   int64_t nzu = 0, nzh = 0, nwarps = 0, nctas = 0, nslots = 0, zpart_len = 0;
   size_t bytes() const {
     return zu.bytes() + zh.bytes() + zw.bytes() + zhw.bytes() + zgroups.bytes() + zcnt.bytes() + chunks.bytes() +
-           portions.bytes() + cta_first.bytes() + rgroups.bytes() + rcnt.bytes() + ypart.bytes() + err.bytes();
+           portions.bytes() + cta_first.bytes() + rgroups.bytes() + rcnt.bytes() + ypart.bytes();
   }
 };
 
@@ -219,8 +218,6 @@ void plan_stream(HMatrix& H, const std::vector<FarUnit>& units, const std::vecto
                  const std::vector<FarGroup>& ugroups, const std::vector<int32_t>& seg, const std::vector<int64_t>& ip,
                  const std::vector<int64_t>& hb, const std::vector<int64_t>& nb, const std::vector<RowItem>& items,
                  cudaStream_t s);
-// the timeout code of an apply kernel since the last call, or 0
-int stream_error(HMatrix& H, cudaStream_t s);
 
 // tensor-core far field of the multi-state apply (hmat_tc.cu): tc_build packs the factors
 // (needs the FP64 pools), tc_far_apply returns the far part of Y (perm order, [Nb][8] FP64)

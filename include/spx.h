@@ -210,8 +210,7 @@ SPX_API int spx_hmat_apply_multi(spx_hmat h, const double* X, double* Y, int32_t
  * rounded to FP32 whatever the packing (with an FP64 packing the tensor-core far field is
  * that of the FP32 packing).  Needs the H-matrix's FP64 factors (built or imported, not
  * merged); spx_hmat_recompress drops the plan.  spx_hmat_tc_status returns (and clears) the
- * timeout flag of its kernels and of the single-vector apply (SPX_ERR_TIMEOUT if a bounded wait
- * ran out, else SPX_OK). */
+ * timeout flag of its kernels (SPX_ERR_TIMEOUT if a bounded wait ran out, else SPX_OK). */
 /* enable = 2 autotunes: one 8-state apply is timed on the CUDA-core kernels and on tensor-core
  * tiles of 512 and of 2048 K elements, and the fastest is kept (*plan_bytes = 0 when the
  * CUDA cores win). */
