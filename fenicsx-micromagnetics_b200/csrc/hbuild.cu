@@ -343,6 +343,26 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
   DevBuf<AcaDesc> dad, dupd;
   DevBuf<AcaState> dst;
   DevBuf<Partial> dpart;
+  // room in a pool; when it cannot grow, the workspace goes first (before a batch all of it, which
+  // the next batch allocates again; at its end A, which only the updates use, and what UV holds
+  // beyond the batch's `uv` entries)
+  auto reserve = [&](GrowBuf& g, int64_t n, int64_t uv) {
+    try {
+      return g.reserve(n);
+    } catch (const Error& e) {
+      if (e.code != ERR_OOM || A.n + UV.n == 0) throw;
+      (void)cudaGetLastError();  // the failed allocation is dealt with here
+    }
+    A.release();
+    if (uv == 0) {
+      UV.release();
+    } else if (static_cast<int64_t>(UV.n) > uv) {
+      DevBuf<double> keep(uv);
+      SPX_CUDA(cudaMemcpy(keep.p, UV.p, uv * sizeof(double), cudaMemcpyDeviceToDevice));
+      UV = std::move(keep);
+    }
+    return g.reserve(n);
+  };
   auto room = [](auto& b, int64_t n) {
     if (static_cast<int64_t>(b.n) < n) {
       b.release();
@@ -396,7 +416,7 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
       std::vector<int64_t> offs;
       for (auto& pr : nearl) {
         const TreeNode &R = nodes[pr.first], &C = nodes[pr.second];
-        offs.push_back(near_g.reserve((int64_t)R.size() * C.size()));
+        offs.push_back(reserve(near_g, (int64_t)R.size() * C.size(), 0));
       }
       for (size_t q = 0; q < nearl.size(); ++q) {
         const TreeNode &R = nodes[nearl[q].first], &C = nodes[nearl[q].second];
@@ -532,10 +552,10 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
         else dec = 2;
         decision[bq] = dec;
         if (dec == 1) {
-          du[bq] = far_g.reserve((int64_t)st.k * d.m);
-          dv[bq] = far_g.reserve((int64_t)st.k * d.n);
+          du[bq] = reserve(far_g, (int64_t)st.k * d.m, uv_tot);
+          dv[bq] = reserve(far_g, (int64_t)st.k * d.n, uv_tot);
         } else if (dec == 2) {
-          dn[bq] = near_g.reserve((int64_t)d.m * d.n);
+          dn[bq] = reserve(near_g, (int64_t)d.m * d.n, uv_tot);
         }
       }
       std::vector<CopyJob> jobs;
