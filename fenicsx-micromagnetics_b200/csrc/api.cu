@@ -135,7 +135,7 @@ struct DemagImpl : DemagBase {
       d.field(reinterpret_cast<TV*>(H), s);
     } else {
       const int64_t n3 = 3 * d.N;
-      if (!tm.n) { tm.alloc(n3); th.alloc(n3); }
+      if (!th.n) { tm.alloc(n3); th.alloc(n3); }
       convert<double, TV>(n3, m, tm.p, s);
       d.potential(tm.p, s, true);
       d.field(th.p, s);
@@ -150,7 +150,7 @@ struct DemagImpl : DemagBase {
     if (sizeof(TV) == sizeof(double))
       return demag_energy<TV, TM>(d, reinterpret_cast<const TV*>(m), reinterpret_cast<const TV*>(H), s);
     const int64_t n3 = 3 * d.N;
-    if (!tm.n) { tm.alloc(n3); th.alloc(n3); }
+    if (!th.n) { tm.alloc(n3); th.alloc(n3); }
     convert<double, TV>(n3, m, tm.p, s);
     convert<double, TV>(n3, H, th.p, s);
     return demag_energy<TV, TM>(d, tm.p, th.p, s);
@@ -213,7 +213,7 @@ struct DemagImpl : DemagBase {
       d.apply_transpose(reinterpret_cast<const TV*>(w), reinterpret_cast<TV*>(out), false, -1, s);
     } else {
       const int64_t n3 = 3 * d.N;
-      if (!tm.n) { tm.alloc(n3); th.alloc(n3); }
+      if (!th.n) { tm.alloc(n3); th.alloc(n3); }
       convert<double, TV>(n3, w, tm.p, s);
       d.apply_transpose(tm.p, th.p, false, -1, s);
       convert<TV, double>(n3, th.p, out, s);

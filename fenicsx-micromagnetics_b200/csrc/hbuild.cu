@@ -351,7 +351,6 @@ void HMatrix::build(const BoundaryDev& bd, const HBuildConfig& c, cudaStream_t s
       return g.reserve(n);
     } catch (const Error& e) {
       if (e.code != ERR_OOM || A.n + UV.n == 0) throw;
-      (void)cudaGetLastError();  // the failed allocation is dealt with here
     }
     A.release();
     if (uv == 0) {

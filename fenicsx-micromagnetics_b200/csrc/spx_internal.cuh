@@ -86,11 +86,16 @@ struct DevBuf {
   ~DevBuf() { release(); }
   void alloc(size_t count) {
     release();
-    n = count;
     if (count) {
       injected_alloc_failure(count * sizeof(T));
-      SPX_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T)));
+      const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&p), count * sizeof(T));
+      if (e != cudaSuccess) {
+        p = nullptr;
+        (void)cudaGetLastError();  // reported here, not by the next launch's check
+        SPX_CUDA(e);
+      }
     }
+    n = count;  // a buffer whose allocation failed stays empty: callers allocate by n
   }
   void release() {
     if (p) cudaFree(p);
