@@ -66,7 +66,7 @@ void BoundaryDev::fill_block(const int32_t* rows_dev, int64_t m, const int32_t* 
                              double* out, cudaStream_t s) const {
   if (m <= 0 || n <= 0) return;
   FillDesc d{0, 0, 0, static_cast<int32_t>(m), static_cast<int32_t>(n)};
-  const int64_t ntiles = fill_tiles(m, n);
+  const int64_t ntiles = fill_tiles(m, n, FILL_TR_BLOCK);
   DevBuf<FillDesc> dd(1);
   DevBuf<int64_t> ts(1);
   int64_t zero = 0;

@@ -13,11 +13,13 @@ struct FillDesc {
   int64_t cols_off;  // offset into cols pool
   int32_t m, n;
 };
-constexpr int FILL_TR = 32, FILL_TC = 32;  // rows and columns of a fill tile
-inline int64_t fill_tiles(int64_t m, int64_t n) {
-  return ((m + FILL_TR - 1) / FILL_TR) * ((n + FILL_TC - 1) / FILL_TC);
+// rows of a fill tile: the blocks of an H-matrix, one block of its own (lindholm.cu); its columns
+constexpr int FILL_TR = 32, FILL_TR_BLOCK = 128, FILL_TC = 32;
+inline int64_t fill_tiles(int64_t m, int64_t n, int tr = FILL_TR) {
+  return ((m + tr - 1) / tr) * ((n + FILL_TC - 1) / FILL_TC);
 }
-// place: position of every boundary node in cols_pool when that is a permutation of them, or null
+// place: position of every boundary node in cols_pool when that is a permutation of them (tiles of
+// FILL_TR rows), or null (tiles of FILL_TR_BLOCK rows)
 void launch_fill(const FillDesc* d_blocks, const int64_t* d_tile_start, int nb, int64_t ntiles,
                  const int32_t* rows_pool, const int32_t* cols_pool, const double* Xb,
                  const int32_t* tri_lid, const double* T, const int32_t* inc_ptr,

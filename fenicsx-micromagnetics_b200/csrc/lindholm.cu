@@ -4,16 +4,19 @@
 // (solid angle via atan2, edge logs via log1p with the 1e-300 floor, opposite-edge
 // convention) and of the block fill of lindholm_hmatrix_gpu/entry_provider.py:41-117.
 //
-// Fill design.  A warp owns a tile of TR=32 block rows x TC=32 block columns.  Its threads
-// build the list of triangles incident to the tile's columns (each triangle kept once, by
-// its lowest in-tile column, in a fixed order so results are deterministic; a triangle's
-// columns found by the node's place in the permutation where the columns are a stretch of
-// it), then every thread (one per row) walks that list, evaluates the three weights once
-// per (row, triangle) and adds them to its private row of a shared-memory accumulator.
-// Bound by FP64 arithmetic (about 500 operations a weight triple).  Rows of a leaf block are
-// about 40, so tiles of 128 rows left two thirds of the threads idle there.  With the lookup in
-// place of a search by compares: 5.8 -> 5.0 ms (4,994 rows), 55.8 -> 49.9 ms (20,802 rows), both
-// changes together.  Triangles incident to the row vertex are skipped (incident_policy
+// Fill design.  A CTA owns a tile of TR block rows x TC=32 block columns.  Its first 32
+// threads build the list of triangles incident to the tile's columns (each triangle kept
+// once, by its lowest in-tile column, in a fixed order so results are deterministic; a
+// triangle's columns found by the node's place in the permutation where the columns are a
+// stretch of it), then every thread (one per row) walks that list, evaluates the three weights
+// once per (row, triangle) and adds them to its private row of a shared-memory accumulator.
+// Bound by FP64 arithmetic (about 500 operations a weight triple).  TR = 32 (a warp) for the
+// blocks of an H-matrix: rows of a leaf block are about 40, so tiles of 128 rows left two thirds
+// of the threads idle there; with the lookup in place of a search by compares 5.8 -> 5.0 ms
+// (4,994 rows), 55.8 -> 49.9 ms (20,802 rows), both changes together.  TR = 128 for a block of
+// its own (the dense operator, a caller's rows and columns), whose list is then built for four
+// times the rows: dense operator of 1,202, 4,994 and 13,442 rows 0.41, 3.22, 21.4 ms (with 32
+// rows 0.45, 3.33, 22.0).  Triangles incident to the row vertex are skipped (incident_policy
 // "skip", gpu/fields/Demag_Lindholm.py:87-96).  The tile is written back row-major with
 // consecutive threads on consecutive columns.  No atomics.
 #include <cmath>
@@ -78,7 +81,8 @@ __global__ void k_lindholm_pairs(int64_t P, const double* __restrict__ x0, const
 }
 
 // tile_start[b] = first task of block b (prefix sum of ceil(m/TR)*ceil(n/TC)); nb blocks
-__global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
+template <int TR>
+__global__ void __launch_bounds__(TR) k_fill_tiles(
     const FillDesc* __restrict__ blocks, const int64_t* __restrict__ tile_start, int nb,
     const int32_t* __restrict__ rows_pool, const int32_t* __restrict__ cols_pool,
     const double* __restrict__ Xb, const int32_t* __restrict__ tri_lid,
@@ -87,7 +91,7 @@ __global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
     double* __restrict__ out) {
   extern __shared__ double smem[];
   double* acc = smem;                                                       // [TR][TC+1]
-  int32_t* scol = reinterpret_cast<int32_t*>(acc + FILL_TR * (FILL_TC + 1));  // [TC]
+  int32_t* scol = reinterpret_cast<int32_t*>(acc + TR * (FILL_TC + 1));  // [TC]
   int32_t* scnt = scol + FILL_TC;                                            // [TC]
   int32_t* stri = scnt + FILL_TC;                                            // [TC*maxinc]
   int32_t* sslot = stri + FILL_TC * maxinc;                                  // [TC*maxinc] packed slots
@@ -103,7 +107,7 @@ __global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
   const int64_t local = task - tile_start[lo];
   const int ntc = (bd.n + FILL_TC - 1) / FILL_TC;
   const int rt = static_cast<int>(local / ntc), ct = static_cast<int>(local % ntc);
-  const int row0 = rt * FILL_TR, col0 = ct * FILL_TC;
+  const int row0 = rt * TR, col0 = ct * FILL_TC;
   const int tc = min(FILL_TC, bd.n - col0);
   const int tid = threadIdx.x;
 
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
     int32_t cv = (tid < tc) ? cols_pool[bd.cols_off + col0 + tid] : -1;
     scol[tid] = (cv >= 0 && cv < Nb) ? cv : -1;  // out-of-range column ids contribute nothing
   }
-  for (int i = tid; i < FILL_TR * (FILL_TC + 1); i += blockDim.x) acc[i] = 0.0;
+  for (int i = tid; i < TR * (FILL_TC + 1); i += blockDim.x) acc[i] = 0.0;
   __syncthreads();
   if (tid < FILL_TC) {
     int cnt = 0;
@@ -167,7 +171,7 @@ __global__ void __launch_bounds__(FILL_TR) k_fill_tiles(
     }
   }
   __syncthreads();
-  const int tr = min(FILL_TR, bd.m - row0);
+  const int tr = min(TR, bd.m - row0);
   for (int idx = tid; idx < tr * FILL_TC; idx += blockDim.x) {
     const int rr = idx / FILL_TC, cc = idx % FILL_TC;
     if (cc < tc) out[bd.out_off + (int64_t)(row0 + rr) * bd.n + col0 + cc] = acc[rr * (FILL_TC + 1) + cc];
@@ -179,8 +183,22 @@ __global__ void k_add_diag(int64_t Nb, const double* __restrict__ omega_sum, dou
   if (i < Nb) B[i * Nb + i] += omega_sum[i] * (1.0 / (4.0 * 3.141592653589793)) - 1.0;
 }
 
-size_t fill_smem_bytes(int maxinc) {
-  return sizeof(double) * FILL_TR * (FILL_TC + 1) + sizeof(int32_t) * (2 * FILL_TC + 2 * FILL_TC * maxinc);
+template <int TR>
+void launch_fill_tiles(const FillDesc* d_blocks, const int64_t* d_tile_start, int nb, int64_t ntiles,
+                       const int32_t* rows_pool, const int32_t* cols_pool, const double* Xb, const int32_t* tri_lid,
+                       const double* T, const int32_t* inc_ptr, const int32_t* inc_tri, const int32_t* place,
+                       int maxinc, int64_t Nb, double* out, cudaStream_t s) {
+  const size_t smem = sizeof(double) * TR * (FILL_TC + 1) + sizeof(int32_t) * (2 * FILL_TC + 2 * FILL_TC * maxinc);
+  static bool attr_set = false;
+  if (!attr_set) {
+    SPX_CUDA(cudaFuncSetAttribute(k_fill_tiles<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    attr_set = true;
+  }
+  SPX_CHECK(smem <= 160 * 1024, "too many incident triangles per boundary vertex for the fill kernel");
+  SPX_CHECK(ntiles < (1ll << 31), "fill launch too large; split the batch");
+  k_fill_tiles<TR><<<static_cast<unsigned>(ntiles), TR, smem, s>>>(
+      d_blocks, d_tile_start, nb, rows_pool, cols_pool, Xb, tri_lid, T, inc_ptr, inc_tri, place, maxinc, Nb, out);
+  SPX_LAUNCH_CHECK();
 }
 
 // Host launcher: fill nb blocks described by host descriptors (device pools given).
@@ -189,20 +207,9 @@ void launch_fill(const FillDesc* d_blocks, const int64_t* d_tile_start, int nb, 
                  const int32_t* tri_lid, const double* T, const int32_t* inc_ptr,
                  const int32_t* inc_tri, const int32_t* place, int maxinc, int64_t Nb, double* out, cudaStream_t s) {
   if (ntiles <= 0) return;
-  const size_t smem = fill_smem_bytes(maxinc);
-  static bool attr_set = false;
-  if (!attr_set) {
-    SPX_CUDA(cudaFuncSetAttribute(k_fill_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    attr_set = true;
-  }
-  SPX_CHECK(smem <= 160 * 1024, "too many incident triangles per boundary vertex for the fill kernel");
-  SPX_CHECK(ntiles < (1ll << 31), "fill launch too large; split the batch");
-  {
-    k_fill_tiles<<<static_cast<unsigned>(ntiles), FILL_TR, smem, s>>>(
-        d_blocks, d_tile_start, nb, rows_pool, cols_pool, Xb, tri_lid, T, inc_ptr, inc_tri, place, maxinc, Nb,
-        out);
-    SPX_LAUNCH_CHECK();
-  }
+  auto go = place ? launch_fill_tiles<FILL_TR> : launch_fill_tiles<FILL_TR_BLOCK>;
+  go(d_blocks, d_tile_start, nb, ntiles, rows_pool, cols_pool, Xb, tri_lid, T, inc_ptr, inc_tri, place, maxinc, Nb, out,
+     s);
 }
 
 void launch_lindholm_pairs(int64_t P, const double* x0, const int32_t* tri, const double* T, int64_t Nt, double* w,
