@@ -271,7 +271,8 @@ __global__ void k_extrap(int64_t n, ExtrapArgs a, T* __restrict__ out) {
 // one reduction).
 //
 // What bounds it: a solve takes tens of iterations of 10^3 to 10^5 rows, so the barriers and
-// the load chain between them, not bytes.  The matrix stays in shared memory for the solve.
+// the load chain between them, not bytes.  The matrix stays in shared memory for the solve (but on
+// the largest systems).
 //   * A system whose matrix and vectors fit the shared memory of one CTA, or of a cluster of up
 //     to eight, runs there: hardware barriers (40 and 450 cycles against 2,600 over the grid), an
 //     update and a product phase per iteration, the residual gathered from (distributed) shared
@@ -280,11 +281,28 @@ __global__ void k_extrap(int64_t n, ExtrapArgs a, T* __restrict__ out) {
 //     and multiplying, every row forms its neighbours' new residuals itself,
 //       r_j' = r_j - alpha (s_j + beta q_j),   s_i' = sum_j a_ij r_j',
 //     from the records {r, s, q} of the last phase (one 16-byte FP32 gather per entry, two
-//     buffers), which saves one of two grid barriers.  Slices past the shared memory stream
-//     through L2.
+//     buffers), which saves one of two grid barriers.
+//   * Where the records' bytes cost more than the barrier, on the grid in two phases again, with
+//     plain vectors (four or eight bytes per gather, most of them in the L1 cache, which no
+//     matrix takes) and twice the warps.  1.03 million nodes off the lattice: FP32 43 us an iteration
+//     (120 with records, whose matrix streams through L2), FP64 59 (160).
 constexpr int CG_BLOCK = 512;
+constexpr int CG_BLOCK_LARGE = 1024;  // TEAM_GRID_LARGE
 constexpr int CG_DYN_MAX = 220 * 1024;
 constexpr int CG_SLICES_PER_CTA = 16;  // CTAs of a cluster: one per 16 slices (a round of its warps)
+// Where TEAM_GRID is the faster form on the grid, by the entries and slices of a CTA: in FP32 as far
+// as its shared memory holds the matrix and its 16 warps go over five rounds of slices, in FP64 (records
+// of 32 bytes) for fewer entries.  us per iteration with TEAM_GRID / TEAM_GRID_LARGE by 10^3 entries and
+// slices of a CTA: FP32 8 and 15 5.3 / 7.5, 15 and 32 6.5 / 7.8, 23 and 48 8.1 / 9.8 (nodes off the lattice, 15
+// entries a row); 11 and 48 6.7 / 8.7, 17 and 76 8.7 / 10.5, 16 and 72 9.8 / 9.9, 19 and 86 11.3 / 9.8, 25 and 113
+// 13.9 / 12.3 (on it, 7 entries a row).  FP64 8 k 7.0 / 8.2, 10 k 9.5 / 8.1, 15 k 12.4 / 8.6 (off the lattice);
+// 7 k 6.9 / 7.5, 11 k 8.8 / 9.3, 17 k 12.5 / 11.7 (on it).
+template <class TM>
+constexpr int64_t cg_record_entries() {
+  return sizeof(TM) == sizeof(float) ? 27000 : 8000;
+}
+constexpr int64_t CG_RECORD_SLICES = 80;
+static_assert(27000 * 8 + (CG_RECORD_SLICES + 8) * 4 <= CG_DYN_MAX, "entries and slice bounds of a CTA");
 
 extern __shared__ __align__(16) unsigned char cg_smem[];
 
@@ -326,7 +344,7 @@ struct CgParams {
   const TV* b;
   TV* x;
   double *bh, *y;
-  TM *p, *d;
+  TM *p, *d, *r, *s, *q;  // r, s, q: TEAM_GRID_LARGE; in records g0, g1: TEAM_GRID
   typename CgRec<TM>::Store *g0, *g1;
   double* part;
   unsigned int* bar;
@@ -338,42 +356,38 @@ struct CgParams {
   double rtol, atol, inner_rtol;
   int maxit, max_outer, warm, project;
   int bh_given;     // bh already holds the scaled, projected right-hand side (FP64)
-  int32_t off_cap;  // slice bounds kept in shared memory (0: read from sp)
+  int32_t off_cap;  // slice bounds kept in shared memory (none by TEAM_GRID_LARGE)
   int32_t cap;      // entries kept in shared memory per CTA
   int32_t rows;     // rows of the largest block (CTA and cluster teams)
 };
 
 template <class TV, class TM, int TEAM>
-__global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgParams<TV, TM> P) {
+__global__ void __launch_bounds__(TEAM == TEAM_GRID_LARGE ? CG_BLOCK_LARGE : CG_BLOCK, 1) k_cg(const __grid_constant__ CgParams<TV, TM> P) {
   using Rec = CgRec<TM>;
-  constexpr bool SM = TEAM != TEAM_GRID;  // records in shared memory
+  constexpr bool SM = TEAM == TEAM_CTA || TEAM == TEAM_CLUSTER;  // vectors in shared memory
+  constexpr bool REC = TEAM == TEAM_GRID;                        // r, s, q in records
+  constexpr bool LARGE = TEAM == TEAM_GRID_LARGE;                // nothing in shared memory
   constexpr int U = sizeof(TM) == 4 ? 8 : 4;  // records in flight per row (grid)
   __shared__ TeamShared S;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int64_t n = P.n;
   if (TEAM == TEAM_CLUSTER) cluster_sync_all();  // every CTA runs before the first remote store
-  // this CTA's block of slices; bounds, values, columns in shared memory as far as they fit
+  // this CTA's block of slices; bounds, values and columns in shared memory (not LARGE)
   const int64_t s0 = P.nslices * blockIdx.x / gridDim.x;
   const int cnt = static_cast<int>(P.nslices * (blockIdx.x + 1) / gridDim.x - s0);
   const int64_t base = P.sp[s0];
   int32_t* soff = reinterpret_cast<int32_t*>(cg_smem);
   TM* sval = reinterpret_cast<TM*>(cg_smem + static_cast<size_t>(P.off_cap) * 4);
   int32_t* scol = reinterpret_cast<int32_t*>(sval + P.cap);
-  const bool off_in = SM || P.off_cap > 0;
   TM* vr = reinterpret_cast<TM*>(scol + P.cap);
   TM *vs = vr + P.rows, *vq = vs + P.rows, *vp = vq + P.rows, *vd = vp + P.rows;
   const unsigned ar = static_cast<unsigned>(__cvta_generic_to_shared(vr));
-  int nres = 0;  // resident slices
-  if (off_in) {
+  if constexpr (LARGE) {
+    vr = P.r; vs = P.s; vq = P.q; vp = P.p; vd = P.d;
+  } else {
     for (int k = threadIdx.x; k <= cnt; k += blockDim.x) soff[k] = static_cast<int32_t>(P.sp[s0 + k] - base);
     __syncthreads();
-    int lo = 0, hi = cnt;  // last bound within the capacity
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (soff[mid] <= P.cap) lo = mid; else hi = mid - 1;
-    }
-    nres = lo;
-    const int m = soff[nres];
+    const int m = soff[cnt];
     for (int k = threadIdx.x; k < m; k += blockDim.x) {
       sval[k] = P.val[base + k];
       int32_t c = P.col[base + k];
@@ -384,16 +398,16 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
       }
       scol[k] = c;
     }
+    __syncthreads();
   }
-  __syncthreads();
   auto bounds = [&](int k, int64_t& o, int& width) {
-    if (off_in) {
-      o = soff[k];
-      width = (soff[k + 1] - soff[k]) >> 5;
-    } else {
+    if constexpr (LARGE) {
       const int64_t a = P.sp[s0 + k];
       o = a - base;
       width = static_cast<int>((P.sp[s0 + k + 1] - a) >> 5);
+    } else {
+      o = soff[k];
+      width = (soff[k + 1] - soff[k]) >> 5;
     }
   };
 #define CG_ROWS_BEGIN                       \
@@ -466,8 +480,8 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
           r64 -= acc + acc2;
         }
         rh += dg * r64 * r64;
-        if constexpr (SM) {
-          const int row = 32 * k + lane;
+        if constexpr (!REC) {
+          const int64_t row = SM ? 32 * k + lane : i;
           vr[row] = static_cast<TM>(r64);
           vs[row] = vq[row] = vp[row] = vd[row] = TM(0);
         } else {
@@ -502,10 +516,10 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
     TM a = TM(0), bt = TM(0);
     for (int it = -1;; ++it) {  // it = -1 (a = bt = 0) only multiplies: s = A r
       double gm = 0.0, dl = 0.0;
-      if constexpr (SM) {
+      if constexpr (!REC) {
         if (it >= 0) {
           CG_ROWS_BEGIN
-            const int row = 32 * k + lane;
+            const int64_t row = SM ? 32 * k + lane : i;
             const TM qn = vs[row] + bt * vq[row], pn = vr[row] + bt * vp[row];
             vq[row] = qn;
             vp[row] = pn;
@@ -515,22 +529,48 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
           if (!team_barrier<TEAM>(P.bar, P.err)) return;
         }
         CG_ROWS_BEGIN
-          const int row = 32 * k + lane, o = soff[k], width = (soff[k + 1] - o) >> 5, so = o + lane;
+          const int64_t row = SM ? 32 * k + lane : i;
+          int64_t o;
+          int width;
+          bounds(k, o, width);
           TM acc = TM(0), acc2 = TM(0);
-          for (int j = 0; j < width; j += 8) {
-            unsigned c[8];
-            TM g[8];
+          if constexpr (SM) {
+            const int so = static_cast<int>(o) + lane;
+            for (int j = 0; j < width; j += 8) {
+              unsigned c[8];
+              TM g[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) c[u] = j + u < width ? static_cast<unsigned>(scol[so + (j + u) * 32]) : ar;
+              for (int u = 0; u < 8; ++u) c[u] = j + u < width ? static_cast<unsigned>(scol[so + (j + u) * 32]) : ar;
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (j + u < width) g[u] = team_load<TEAM>(c[u], TM(0));
+              for (int u = 0; u < 8; ++u)
+                if (j + u < width) g[u] = team_load<TEAM>(c[u], TM(0));
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (j + u < width) {
-                if (u & 1) acc2 += sval[so + (j + u) * 32] * g[u];
-                else acc += sval[so + (j + u) * 32] * g[u];
+              for (int u = 0; u < 8; ++u)
+                if (j + u < width) {
+                  if (u & 1) acc2 += sval[so + (j + u) * 32] * g[u];
+                  else acc += sval[so + (j + u) * 32] * g[u];
+                }
+            }
+          } else {
+            const TM* gv = P.val + base + o + lane;
+            const int32_t* gc = P.col + base + o + lane;
+            for (int j = 0; j < width; j += 8) {
+              int32_t c[8];
+              TM w[8], g[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                const bool in = j + u < width;
+                c[u] = in ? gc[(j + u) * 32] : 0;
+                w[u] = in ? gv[(j + u) * 32] : TM(0);
               }
+#pragma unroll
+              for (int u = 0; u < 8; ++u) g[u] = j + u < width ? vr[c[u]] : TM(0);
+#pragma unroll
+              for (int u = 0; u < 8; u += 2) {
+                acc += w[u] * g[u];
+                acc2 += w[u + 1] * g[u + 1];
+              }
+            }
           }
           const TM sn = acc + acc2;
           vs[row] = sn;
@@ -548,23 +588,20 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
           int width;
           bounds(k, o, width);
           TM acc = TM(0), acc2 = TM(0);
-          const bool res = k < nres;
-          const TM* gv = P.val + base + o + lane;
-          const int32_t* gc = P.col + base + o + lane;
-          const int so = (res ? static_cast<int>(o) : 0) + lane;
+          const int so = static_cast<int>(o) + lane;
           for (int j = 0; j < width; j += U) {
             int32_t c[U];
             Rec g[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-              c[u] = j + u < width ? (res ? scol[so + (j + u) * 32] : gc[(j + u) * 32]) : 0;
+              c[u] = j + u < width ? scol[so + (j + u) * 32] : 0;
 #pragma unroll
             for (int u = 0; u < U; ++u)
               if (j + u < width) g[u] = Rec::load(cur + c[u]);
 #pragma unroll
             for (int u = 0; u < U; ++u)
               if (j + u < width) {
-                const TM w = res ? sval[so + (j + u) * 32] : gv[(j + u) * 32];
+                const TM w = sval[so + (j + u) * 32];
                 const TM rj = g[u].r - a * (g[u].s + bt * g[u].q);
                 if (u & 1) acc2 += w * rj; else acc += w * rj;
               }
@@ -591,8 +628,7 @@ __global__ void __launch_bounds__(CG_BLOCK, 1) k_cg(const __grid_constant__ CgPa
       ginv = 1.0 / gm;
     }
     CG_ROWS_BEGIN
-      if constexpr (SM) P.y[i] += static_cast<double>(vd[32 * k + lane]);
-      else P.y[i] += static_cast<double>(P.d[i]);
+      P.y[i] += static_cast<double>(SM ? vd[32 * k + lane] : P.d[i]);
     CG_ROWS_END
     if (!team_barrier<TEAM>(P.bar, P.err)) return;
   }
@@ -630,7 +666,8 @@ template <class TV, class TM>
 const void* cg_kernel(int team) {
   return team == TEAM_CTA ? reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_CTA>)
          : team == TEAM_CLUSTER ? reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_CLUSTER>)
-                                : reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_GRID>);
+         : team == TEAM_GRID    ? reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_GRID>)
+                                : reinterpret_cast<const void*>(k_cg<TV, TM, TEAM_GRID_LARGE>);
 }
 
 // number of identical diagonal blocks of the FEM system when every sample of an ensemble has
@@ -758,19 +795,28 @@ void CgSystem<TM>::setup(const HostSell& s, const std::vector<double>& vals_sell
     smem_bytes = static_cast<size_t>(small_bytes());
     threads = 32 * static_cast<int>(std::min<int64_t>(CG_BLOCK / 32, std::max<int64_t>(cnt, 4)));
   } else {
+    auto grid_blocks = [&](int t) {
+      threads = t;
+      blocks(static_cast<int>(std::min<int64_t>((s.nslices + t / 32 - 1) / (t / 32), num_sms(dev))));
+    };
     team = TEAM_GRID;
-    threads = CG_BLOCK;
-    const int64_t per_cta = CG_BLOCK / 32;
-    blocks(static_cast<int>(std::min<int64_t>((s.nslices + per_cta - 1) / per_cta, num_sms(dev))));
-    if (off_cap * 4 > CG_DYN_MAX / 4) off_cap = 0;  // thousands of slices a CTA: all streamed
-    cap = off_cap ? static_cast<int32_t>(std::min<int64_t>(need, (CG_DYN_MAX - off_cap * 4) / eb / 32 * 32)) : 0;
+    grid_blocks(CG_BLOCK);
     rows = 0;
-    smem_bytes = static_cast<size_t>(off_cap) * 4 + static_cast<size_t>(cap) * eb;
+    if (need <= cg_record_entries<TM>() && cnt <= CG_RECORD_SLICES) {
+      cap = static_cast<int32_t>(need);
+      smem_bytes = static_cast<size_t>(off_cap * 4 + need * eb);
+    } else {
+      team = TEAM_GRID_LARGE;
+      grid_blocks(CG_BLOCK_LARGE);
+      off_cap = cap = 0;
+      smem_bytes = 0;
+    }
   }
   part.alloc(4 * 4 * static_cast<size_t>(std::max(grid, num_sms(dev))));
   std::vector<const void*> ks{cg_kernel<double, TM>(team)};
   if constexpr (sizeof(TM) == sizeof(float)) ks.push_back(cg_kernel<float, TM>(team));
-  for (const void* k : ks) SPX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_DYN_MAX));
+  if (team != TEAM_GRID_LARGE)
+    for (const void* k : ks) SPX_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, CG_DYN_MAX));
 }
 
 template <class TM>
@@ -841,6 +887,9 @@ CgStats CgSystem<TM>::solve(const TV* b, TV* x, double rtol, double atol, int ma
     q.g1 = q.g0 + n;
     q.p = reinterpret_cast<TM*>(q.g1 + n);
     q.d = q.p + n;
+    q.r = reinterpret_cast<TM*>(work.p);  // in place of the records
+    q.s = q.r + n;
+    q.q = q.s + n;
     q.part = part.p; q.bar = bar.p; q.err = err.p; q.iters = iters.p; q.resid = resid.p;
     q.iters_acc = iters_acc.p;
     q.res_acc = res_acc.p;

@@ -7,9 +7,10 @@
 namespace spx {
 
 // The CTAs of a solve: one CTA (TEAM_CTA), one cluster (TEAM_CLUSTER) or the whole cooperative
-// grid (TEAM_GRID).  A barrier costs 1.3 us over the grid, so small systems run on one CTA or
+// grid, in a form with as few barriers as there can be (TEAM_GRID) or with as few bytes
+// (TEAM_GRID_LARGE).  A barrier costs 1.3 us over the grid, so small systems run on one CTA or
 // one cluster, whose barriers are in hardware.
-enum : int { TEAM_CTA = 0, TEAM_CLUSTER = 1, TEAM_GRID = 2 };
+enum : int { TEAM_CTA = 0, TEAM_CLUSTER = 1, TEAM_GRID = 2, TEAM_GRID_LARGE = 3 };
 constexpr int TEAM_MAX_CLUSTER = 8;  // portable cluster size
 
 struct TeamShared {
