@@ -139,7 +139,7 @@ struct CgSystem {
   DevBuf<double> seg_part;    // chunk sums [components][seg_maxch]
   void set_segments(const std::vector<int64_t>& offsets, cudaStream_t s);
   DevBuf<double> pred0, delta;
-  // reduction of one inner solve before its residual is recomputed in FP64
+  // reduction of one inner solve before its residual is recomputed in FP64 (setup: less on large systems)
   double inner_rtol = sizeof(TM) == sizeof(float) ? 1e-3 : 1e-7;
   int max_outer = 10;
   int grid = 0, threads = 0, team = 0;  // CTAs of k_cg, their threads, which kind of team they form
