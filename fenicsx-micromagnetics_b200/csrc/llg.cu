@@ -39,64 +39,92 @@ __global__ void __launch_bounds__(256) k_stage(StageArgs<TV, TM> a) {
     // The DMI form (13 to 16 values an entry) loads the entries in batches of three, every load of
     // a batch in flight before the first sum; summed in order.  64 boxes of 2,646 nodes with DMI and
     // anisotropy, FP32 matrix: 154 -> 78 us (two: 92, four: 102, registers against warps); 200x200x2
-    // film without demag, FP64: 35 -> 32 us.  Without DMI one entry a pass, which the compiler
-    // unrolls: 400x400x2 film 50 us, against 53 to 102 us for batches of three to ten.
-    constexpr int U = DMI ? 3 : 1;
+    // film without demag, FP64: 35 -> 29 us.  Entry by entry, as the compiler unrolls it, without DMI
+    // (400x400x2 film with demag 50 us, 53 to 102 us in batches of three to ten; batches of one cost
+    // small meshes 2 of 6 us) and for an FP32 matrix with FP64 vectors without demag (400x400x2 film
+    // 78 us, 80 in batches).
     const int64_t L = a.L;
-    for (int k = 0; k < width; k += U) {
-      const int64_t i0 = base + ((int64_t)k << 5) + lane;
-      int32_t c[U];
+    if constexpr (DMI && (DEMAG || sizeof(TV) == sizeof(TM))) {
+      constexpr int U = 3;
+      for (int k = 0; k < width; k += U) {
+        const int64_t i0 = base + ((int64_t)k << 5) + lane;
+        int32_t c[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) c[u] = k + u < width ? a.col[i0 + 32 * u] : 0;
-      TV x[U], y[U], z[U], ph[U];
-      TM e[U], kz[U], kd[DMI ? U : 1][9], g[DEMAG ? U : 1][3];
+        for (int u = 0; u < U; ++u) c[u] = k + u < width ? a.col[i0 + 32 * u] : 0;
+        TV x[U], y[U], z[U], ph[U];
+        TM e[U], kz[U], kd[U][9], g[DEMAG ? U : 1][3];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < width) {
-          const int64_t j = c[u], idx = i0 + 32 * u;
-          x[u] = a.m[3 * j];
-          y[u] = a.m[3 * j + 1];
-          z[u] = a.m[3 * j + 2];
-          e[u] = a.Kex[idx];
-          if (a.Kz) kz[u] = a.Kz[idx];
-          if (DMI) {
+        for (int u = 0; u < U; ++u)
+          if (k + u < width) {
+            const int64_t j = c[u], idx = i0 + 32 * u;
+            x[u] = a.m[3 * j];
+            y[u] = a.m[3 * j + 1];
+            z[u] = a.m[3 * j + 2];
+            e[u] = a.Kex[idx];
+            if (a.Kz) kz[u] = a.Kz[idx];
 #pragma unroll
-            for (int q = 0; q < 9; ++q) kd[DMI ? u : 0][q] = a.Kd[q * L + idx];
+            for (int q = 0; q < 9; ++q) kd[u][q] = a.Kd[q * L + idx];
+            if (DEMAG) {
+              ph[u] = a.phi[j];
+#pragma unroll
+              for (int q = 0; q < 3; ++q) g[DEMAG ? u : 0][q] = a.Gv[q * L + idx];
+            }
           }
-          if (DEMAG) {
-            ph[u] = a.phi[j];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) g[DEMAG ? u : 0][q] = a.Gv[q * L + idx];
-          }
-        }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < width) {
-          const TV dx = x[u] - mx, dy = y[u] - my, dz = z[u] - mz;
-          const TV ex = static_cast<TV>(e[u]);
-          hx += ex * dx;
-          hy += ex * dy;
-          hz += ex * dz;
-          if (a.Kz) {
-            const TV w = static_cast<TV>(kz[u]);
-            zx += w * dx;
-            zy += w * dy;
-            zz += w * dz;
-          }
-          if (DMI) {
-            const TM* K = kd[DMI ? u : 0];
+        for (int u = 0; u < U; ++u)
+          if (k + u < width) {
+            const TV dx = x[u] - mx, dy = y[u] - my, dz = z[u] - mz;
+            const TV ex = static_cast<TV>(e[u]);
+            hx += ex * dx;
+            hy += ex * dy;
+            hz += ex * dz;
+            if (a.Kz) {
+              const TV w = static_cast<TV>(kz[u]);
+              zx += w * dx;
+              zy += w * dy;
+              zz += w * dz;
+            }
+            const TM* K = kd[u];
             hx += static_cast<TV>(K[0]) * dx + static_cast<TV>(K[1]) * dy + static_cast<TV>(K[2]) * dz;
             hy += static_cast<TV>(K[3]) * dx + static_cast<TV>(K[4]) * dy + static_cast<TV>(K[5]) * dz;
             hz += static_cast<TV>(K[6]) * dx + static_cast<TV>(K[7]) * dy + static_cast<TV>(K[8]) * dz;
+            if (DEMAG) {
+              const TV p = ph[u] - pi;
+              const TM* G = g[DEMAG ? u : 0];
+              hx += static_cast<TV>(G[0]) * p;
+              hy += static_cast<TV>(G[1]) * p;
+              hz += static_cast<TV>(G[2]) * p;
+            }
           }
-          if (DEMAG) {
-            const TV p = ph[u] - pi;
-            const TM* G = g[DEMAG ? u : 0];
-            hx += static_cast<TV>(G[0]) * p;
-            hy += static_cast<TV>(G[1]) * p;
-            hz += static_cast<TV>(G[2]) * p;
-          }
+      }
+    } else {
+      for (int k = 0; k < width; ++k) {
+        const int64_t idx = base + ((int64_t)k << 5) + lane;
+        const int64_t j = a.col[idx];
+        const TV dx = a.m[3 * j] - mx, dy = a.m[3 * j + 1] - my, dz = a.m[3 * j + 2] - mz;
+        const TV e = static_cast<TV>(a.Kex[idx]);
+        hx += e * dx;
+        hy += e * dy;
+        hz += e * dz;
+        if (a.Kz) {
+          const TV kz = static_cast<TV>(a.Kz[idx]);
+          zx += kz * dx;
+          zy += kz * dy;
+          zz += kz * dz;
         }
+        if (DMI) {
+          const TM* K = a.Kd + idx;
+          hx += static_cast<TV>(K[0]) * dx + static_cast<TV>(K[L]) * dy + static_cast<TV>(K[2 * L]) * dz;
+          hy += static_cast<TV>(K[3 * L]) * dx + static_cast<TV>(K[4 * L]) * dy + static_cast<TV>(K[5 * L]) * dz;
+          hz += static_cast<TV>(K[6 * L]) * dx + static_cast<TV>(K[7 * L]) * dy + static_cast<TV>(K[8 * L]) * dz;
+        }
+        if (DEMAG) {
+          const TV p = a.phi[j] - pi;
+          hx += static_cast<TV>(a.Gv[idx]) * p;
+          hy += static_cast<TV>(a.Gv[a.L + idx]) * p;
+          hz += static_cast<TV>(a.Gv[2 * a.L + idx]) * p;
+        }
+      }
     }
     if (DMI) {
       const double* S = a.Ksum;
@@ -203,47 +231,66 @@ __global__ void __launch_bounds__(256) k_jv(StageArgs<TV, TM> a, const TV* __res
     const TV vx = v[3 * i], vy = v[3 * i + 1], vz = v[3 * i + 2];
     TV hvx = 0, hvy = 0, hvz = 0;
     TV jvx = 0, jvy = 0, jvz = 0;  // Z(v)
-    // batches as in k_stage; 200x200x2 film, FP64: 42 -> 32 us (three: 40, four: 37)
-    constexpr int U = DMI ? 2 : 1;
+    // batches as in k_stage; 200x200x2 film, FP64: 42 -> 32 us (three: 40, four: 37); with an FP32
+    // matrix and FP64 vectors entry by entry (400x400x2 film 80 us, 93 in batches of two, 103 of one)
     const int64_t L = a.L;
-    for (int k = 0; k < width; k += U) {
-      const int64_t i0 = base + ((int64_t)k << 5) + lane;
-      int32_t c[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) c[u] = k + u < width ? a.col[i0 + 32 * u] : 0;
-      TV xs[U], ys[U], zs[U];
-      TM e[U], kzs[U], kd[DMI ? U : 1][9];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < width) {
-          const int64_t j = c[u], idx = i0 + 32 * u;
-          xs[u] = v[3 * j];
-          ys[u] = v[3 * j + 1];
-          zs[u] = v[3 * j + 2];
-          e[u] = a.Kex[idx];
-          if (a.Kz) kzs[u] = a.Kz[idx];
-          if (DMI) {
-#pragma unroll
-            for (int q = 0; q < 9; ++q) kd[DMI ? u : 0][q] = a.Kd[q * L + idx];
-          }
+    if constexpr (DMI && sizeof(TV) != sizeof(TM)) {
+      for (int k = 0; k < width; ++k) {
+        const int64_t idx = base + ((int64_t)k << 5) + lane;
+        const int64_t j = a.col[idx];
+        const TV x = v[3 * j] - vx, y = v[3 * j + 1] - vy, z = v[3 * j + 2] - vz;
+        const TV e = static_cast<TV>(a.Kex[idx]);
+        hvx += e * x; hvy += e * y; hvz += e * z;
+        if (a.Kz) {
+          const TV kz = static_cast<TV>(a.Kz[idx]);
+          jvx += kz * x; jvy += kz * y; jvz += kz * z;
         }
+        const TM* K = a.Kd + idx;
+        hvx += static_cast<TV>(K[0]) * x + static_cast<TV>(K[L]) * y + static_cast<TV>(K[2 * L]) * z;
+        hvy += static_cast<TV>(K[3 * L]) * x + static_cast<TV>(K[4 * L]) * y + static_cast<TV>(K[5 * L]) * z;
+        hvz += static_cast<TV>(K[6 * L]) * x + static_cast<TV>(K[7 * L]) * y + static_cast<TV>(K[8 * L]) * z;
+      }
+    } else {
+      constexpr int U = DMI ? 2 : 1;
+      for (int k = 0; k < width; k += U) {
+        const int64_t i0 = base + ((int64_t)k << 5) + lane;
+        int32_t c[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < width) {
-          const TV x = xs[u] - vx, y = ys[u] - vy, z = zs[u] - vz;
-          const TV ex = static_cast<TV>(e[u]);
-          hvx += ex * x; hvy += ex * y; hvz += ex * z;
-          if (a.Kz) {
-            const TV kz = static_cast<TV>(kzs[u]);
-            jvx += kz * x; jvy += kz * y; jvz += kz * z;
+        for (int u = 0; u < U; ++u) c[u] = k + u < width ? a.col[i0 + 32 * u] : 0;
+        TV xs[U], ys[U], zs[U];
+        TM e[U], kzs[U], kd[DMI ? U : 1][9];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (k + u < width) {
+            const int64_t j = c[u], idx = i0 + 32 * u;
+            xs[u] = v[3 * j];
+            ys[u] = v[3 * j + 1];
+            zs[u] = v[3 * j + 2];
+            e[u] = a.Kex[idx];
+            if (a.Kz) kzs[u] = a.Kz[idx];
+            if (DMI) {
+#pragma unroll
+              for (int q = 0; q < 9; ++q) kd[DMI ? u : 0][q] = a.Kd[q * L + idx];
+            }
           }
-          if (DMI) {
-            const TM* K = kd[DMI ? u : 0];
-            hvx += static_cast<TV>(K[0]) * x + static_cast<TV>(K[1]) * y + static_cast<TV>(K[2]) * z;
-            hvy += static_cast<TV>(K[3]) * x + static_cast<TV>(K[4]) * y + static_cast<TV>(K[5]) * z;
-            hvz += static_cast<TV>(K[6]) * x + static_cast<TV>(K[7]) * y + static_cast<TV>(K[8]) * z;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (k + u < width) {
+            const TV x = xs[u] - vx, y = ys[u] - vy, z = zs[u] - vz;
+            const TV ex = static_cast<TV>(e[u]);
+            hvx += ex * x; hvy += ex * y; hvz += ex * z;
+            if (a.Kz) {
+              const TV kz = static_cast<TV>(kzs[u]);
+              jvx += kz * x; jvy += kz * y; jvz += kz * z;
+            }
+            if (DMI) {
+              const TM* K = kd[DMI ? u : 0];
+              hvx += static_cast<TV>(K[0]) * x + static_cast<TV>(K[1]) * y + static_cast<TV>(K[2]) * z;
+              hvy += static_cast<TV>(K[3]) * x + static_cast<TV>(K[4]) * y + static_cast<TV>(K[5]) * z;
+              hvz += static_cast<TV>(K[6]) * x + static_cast<TV>(K[7]) * y + static_cast<TV>(K[8]) * z;
+            }
           }
-        }
+      }
     }
     if (DMI) {
       const double* S = a.Ksum;
