@@ -19,7 +19,7 @@
 // What bounds k_pcg_amg is the chain of loads inside each of its 15 or so phases per
 // iteration, not bytes: 148 CTAs sweep 10^3 to 10^6 rows between two grid barriers of 1.3 us.
 // So (1) every CTA owns a contiguous block of slices of each level, and keeps their values,
-// columns and slice bounds in shared memory for the whole solve, as far as 200 KB go (finest
+// columns and slice bounds in shared memory for the whole solve, as far as 220 KB go (finest
 // level first, which five phases of an iteration read): a phase's chain is one gather, and no
 // matrix byte crosses L2 again; slices past that stream from global memory in the same loop;
 // (2) eight gathers of a row are in flight; (3) the level descriptors are kernel parameters;
@@ -566,7 +566,6 @@ __device__ void post_d_r(const AmgLevelDev& L, RowRange rr, const double* __rest
   }
 }
 
-// dense coarsest level for R blocks (interleaved vectors; b entries past nc are taken as 0)
 // the right-hand sides of the dense coarsest level, transposed to [R][nc], for k_pcg_amg_r's
 // coarse phase (dynamic shared memory of nc x R floats)
 extern __shared__ float pcg_coarse_smem[];
@@ -1299,7 +1298,7 @@ __device__ bool vcycle_r(const PcgParams<TV>& P, int slot, double* sh, unsigned 
 
 // k_pcg_amg on R identical blocks: one CG on the block-diagonal system (the scalars are those of
 // the whole system, as for a disjoint union), with the block's matrix and hierarchy stored once.
-// Per-row data (rsum, sdinv, diag, level dinv) are those of block row i (identical blocks); b, x,
+// Per-row data (rsum, diag, level dinv) are those of block row i (identical blocks); b, x,
 // y, bh are indexed in block order (r n + i), the work vectors r, p, q and the level vectors
 // interleaved (i R + r).
 template <class TV, int R>

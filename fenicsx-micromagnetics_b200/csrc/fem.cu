@@ -770,7 +770,7 @@ void CgSystem<TM>::setup(const HostSell& s, const std::vector<double>& vals_sell
   // the grid, a slice a warp.  Per iteration (before: a grid kernel with one or two phases, own
   // vectors and matrix in global memory): 11 slices on one CTA 1.3 us, 46 slices (20x20x5 box) on
   // four 1.8 us (10 us on its two CTAs before; 2.3 on eight, 3.0 on two), 132 slices on eight
-  // 2.9 us (grid 4.7), 428 slices on eight 4.5 us (grid 4.5); the grid 4.3-5 us up to 1,200 slices
+  // 2.9 us (grid 4.7), 428 slices on eight 4.5 us (grid 4.5); the grid 4.4-5.2 us up to 1,600 slices (FP32)
   int64_t cnt = 0, need = 0;  // slices and entries of the largest block
   const int64_t eb = sizeof(TM) + sizeof(int32_t);
   auto blocks = [&](int g) {

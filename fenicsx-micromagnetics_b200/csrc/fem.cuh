@@ -2,7 +2,7 @@
 //
 // Precision: DemagCtx<TV, TM> keeps nodal vectors (m, u1, u2, phi, b, g) in TV and the large
 // matrices (Div, G/V, the CG values) in TM.
-//   <double, double>  FP64 everywhere, pipelined FP64 CG
+//   <double, double>  FP64 everywhere
 //   <float,  float>   plain FP32 (FP32 CG inside FP64 iterative refinement, FP32 vectors)
 //   <double, float>   mixed: FP64 vectors, FP32 matrices, FP32 inner CG + FP64 refinement
 // Operators whose rows sum to zero (G, exchange) are applied in difference form
@@ -104,11 +104,8 @@ struct CgSystem {
   // FP64 data of the refinement solve: values, solution state and right-hand side are those of
   // the scaled system for k_cg, unscaled for the AMG PCG
   DevBuf<double> vals64, sdinv64, diag64, y64, bh64;
-  DevBuf<TM> sdinv;    // 1/sqrt(d) (pipelined FP64 path)
-  DevBuf<TM> diag;
   DevBuf<char> work;   // solver vectors
-  DevBuf<double> part;  // per-CTA partial sums [3 slots][grid][4]
-  DevBuf<double> red;   // scalars
+  DevBuf<double> part;  // per-CTA partial sums
   DevBuf<unsigned int> bar;
   DevBuf<int> err;
   DevBuf<int> iters;
@@ -128,7 +125,7 @@ struct CgSystem {
   // stage correction: slots 1..3 add slot 0's last prediction error (solution - guess)
   bool stage_correct = false, have_pred0 = false, have_delta = false;
   // kind of the last solve (0 forward, 1 adjoint, 2 tangent): a warm start from the solver
-  // state (y64 or x) is taken only from a solve of the same kind, whose right-hand sides
+  // state (y64) is taken only from a solve of the same kind, whose right-hand sides
   // have the same scale; otherwise the solve starts from zero
   int last_kind = 0;
   // singular systems made of several independent components (ensembles): node offsets of
@@ -167,10 +164,6 @@ struct CgSystem {
   template <class TV>
   CgStats solve(const TV* b, TV* x, double rtol, double atol, int maxit, bool warm, bool project, int slot,
                 cudaStream_t st, bool sync_stats, int kind = -1);
-  void reset_history() {
-    for (int s = 0; s < CG_SLOTS; ++s) hcount[s] = hhead[s] = 0;
-    have_pred0 = have_delta = false;
-  }
 };
 
 // Block-diagonal boundary operator of an ensemble (a disjoint union of independent sample

@@ -160,17 +160,17 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// What bounds the apply: HBM reads in flight, not arithmetic (replacing the FMAs by one XOR per
-// entry changes neither kernel's time).  32 warps per SM with four 16-byte loads of a lane in
-// flight and the next tile of each warp on its way into L2: 148 x 32 x 4 KB = 19 MB, three times
-// what 1 us of latency takes at 6.5 TB/s.  Tiles of 16 KB (77 MB of prefetch, over half of L2)
-// cost FP64 factors 18 % and FP32 ones 1-13 %, 2 KB tiles 6-17 %; three CTAs with six loads a lane
-// FP32 8 %.
+// What bounds the apply: with FP64 factors HBM (film of 400 cubes a side, 13.8 GB: 6.2 TB/s, 0.94 of
+// the copy rate).  FP32 (6.9 GB, 4.8 TB/s) and BF16 factors (about 3.9 GB, 2.8 TB/s) take nearly the
+// same time as each other at that size, so there it goes with the entries, not with the bytes (which
+// part of an entry's chain of loads, conversion and sum is not settled: one XOR in place of the FMAs
+// changes neither kernel's time).  32 warps per SM with four 16-byte loads of a lane in flight and the
+// next tile of each warp on its way into L2.  Tiles of 16 KB cost FP64 factors 18 % and FP32 ones
+// 1-13 %, 2 KB tiles 6-17 %; three CTAs with six loads a lane FP32 8 %.
 // us per product (CTA per row segment, power-of-two lane split, 16 KB units -> this), films of 24,
 // 48, 100, 150, 200, 400 cubes a side: FP32 31.8 -> 24.2, 42.4 -> 29.1, 95 -> 67.6, 167 -> 152,
-// 296 -> 270, 1436 -> 1377..1428; FP64 29.6 -> 23.5, 43.2 -> 29.4, 126 -> 102, 260 -> 230,
-// 465 -> 449, 2359 -> 2295; BF16 28.7 -> 29.6, 44.0 -> 33.5, 86 -> 69, 157 -> 138, 280 -> 249,
-// 1417 -> 1369.
+// 296 -> 270, 1436 -> 1443 (no gain there); FP64 29.6 -> 23.5, 43.2 -> 29.4, 126 -> 102, 260 -> 228,
+// 465 -> 423, 2359 -> 2243; BF16 28.7 -> 29.6, 44.0 -> 33.5, 86 -> 69, 157 -> 138, 280 -> 249, 1417 -> 1384.
 constexpr int ST_WARPS = 8;          // warps per CTA
 constexpr int ST_CTAS_PER_SM = 4;
 constexpr int ST_TILE = 4096;        // bytes of a tile
